@@ -24,6 +24,7 @@ SIGNATURES = {
     "bfp8_last_cuda_error": (_int, []),
     "bfp8_set_weights_at_rest": (_int, [_int]),
     "bfp8_reencode_half": (_int, [_ptr, _ptr, _i64, _ptr, _ptr, _i64, _ptr, _ptr, _ptr]),
+    "bfp8_reencode_half_swiglu": (_int, [_ptr, _ptr, _i64, _i64, _ptr, _ptr, _i64, _ptr, _ptr, _ptr]),
     "bfp8_validate_e4m3": (_int, [_ptr, _i64, _ptr, _i64, _ptr, _ptr]),
     "bfp8_quant_block128_f32": (_int, [_ptr, _i64, _i64, _i64, _ptr, _i64, _ptr, _int, _ptr]),
     "bfp8_quant_act_1x128_bf16": (_int, [_ptr, _i64, _i64, _i64, _ptr, _i64, _ptr, _i64, _i64, _int, _ptr, _ptr]),

@@ -17,7 +17,8 @@ There is no CPU implementation in this package.
 import torch
 
 from . import _lib
-from .fp8_codec import BLOCK, _device_for, _read_status, _status_buffer, _stream_ptr, quantize_act_1x128
+from .fp8_codec import (BLOCK, _device_for, _read_status, _reencode_on_device, _status_buffer, _stream_ptr,
+                        quantize_act_1x128)
 
 # Zero-initialised scratch per (device, stream).  The small-M schedule keeps per-tile arrival counters
 # there and returns them to zero, so one buffer serves every call issued on that stream.
@@ -231,6 +232,14 @@ def prepare_weight_swiglu(weight, scales, native_half=True):
     Re-encodes to the half range when asked (as prepare_weight), then interleaves the rows in chunks of 64
     so a GEMM tile holds both factors of its outputs.  The scale grid keeps its order.  I % 128 == 0.
     """
+    if (native_half and isinstance(weight, torch.Tensor) and weight.ndim == 2 and weight.shape[0] % (2 * BLOCK) == 0
+            and weight.shape[1] % 16 == 0 and weight.numel() < 1 << 36):
+        dev = _device_for(weight, scales)
+        weight = weight.to(dev)
+        if weight.data_ptr() % 16 == 0:
+            # rows of whole 16-byte vectors: re-encoded and put in the GEMM's row order in one pass over the weight
+            codes, scales, _ = _reencode_on_device(weight, scales.to(dev), swiglu_inter=weight.shape[0] // 2)
+            return codes, scales
     codes, scales = prepare_weight(weight, scales, native_half)
     if codes.ndim != 2 or codes.shape[0] % (2 * BLOCK) != 0:
         raise ValueError("fused gate/up weight must be [2 * I, K] with I a multiple of 128")

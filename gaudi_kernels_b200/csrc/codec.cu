@@ -34,10 +34,24 @@ __device__ __forceinline__ void reencode_vec(uint4& v, uint32_t& inexact, uint32
   }
 }
 
+// Where vector i (16 codes) of a fused gate/up weight [2 inter][16 vecs] goes in the order the SwiGLU GEMM reads: chunk c
+// of 64 outputs becomes rows [128 c, 128 c + 64) (gate) and [128 c + 64, 128 c + 128) (up).  32-bit arithmetic: the
+// caller checks that the weight has fewer than 2^32 vectors.
+__device__ __forceinline__ int64_t interleaved_vec(uint32_t i, uint32_t vecs, uint32_t inter) {
+  const uint32_t row = i / vecs, v = i - row * vecs;
+  const uint32_t half = row >= inter ? 64u : 0u, o = row >= inter ? row - inter : row;
+  return static_cast<int64_t>((o & ~63u) * 2u + half + (o & 63u)) * vecs + v;
+}
+
+// kInterleave: `in` is a fused gate/up weight of 2 * inter rows of `vecs` 16-byte vectors and the codes are written in
+// the interleaved row order (both buffers 16-byte aligned, in != out).  Load time is bound by HBM, and re-encoding in one
+// pass and reordering in a second moved every byte twice.
+template <bool kInterleave>
 __global__ void __launch_bounds__(kReencodeThreads)
 reencode_half_kernel(const uint8_t* in, uint8_t* out, int64_t n, int vec_ok,          // in == out is allowed
                      const float* scales_in, float* scales_out, int64_t n_scales,
-                     unsigned long long* __restrict__ rounded, uint32_t* __restrict__ status) {
+                     unsigned long long* __restrict__ rounded, uint32_t* __restrict__ status,
+                     uint32_t vecs, uint32_t inter) {
   __shared__ uint32_t cta_inexact, cta_bad;
   if (threadIdx.x == 0) { cta_inexact = 0; cta_bad = 0; }
   __syncthreads();
@@ -73,11 +87,11 @@ reencode_half_kernel(const uint8_t* in, uint8_t* out, int64_t n, int vec_ok,    
       const int64_t i = chunk + u * kReencodeThreads + threadIdx.x;
       if (i < nvec) {
         reencode_vec(v[u], inexact, bad);
-        __stcs(vout + i, v[u]);
+        __stcs(vout + (kInterleave ? interleaved_vec(static_cast<uint32_t>(i), vecs, inter) : i), v[u]);
       }
     }
     // ragged tail (fewer than 16 bytes): the last CTA's first threads
-    if (blockIdx.x == gridDim.x - 1) {
+    if (!kInterleave && blockIdx.x == gridDim.x - 1) {
       const int64_t i = (nvec << 4) + threadIdx.x;
       if (i < n) {
         const uint32_t c = in[i];
@@ -654,8 +668,29 @@ extern "C" int bfp8_reencode_half(const uint8_t* codes_in, uint8_t* codes_out, i
   const int64_t ctas = (n + per_cta - 1) / per_cta;
   if (ctas > 2147483647LL) return BFP8_ERR_SHAPE;
   const int grid = static_cast<int>(ctas);
-  reencode_half_kernel<<<grid, kReencodeThreads, 0, st>>>(codes_in, codes_out, n, vec_ok, scales_in, scales_out, n_scales,
-                                                          rounded_dev, status_dev);
+  reencode_half_kernel<false><<<grid, kReencodeThreads, 0, st>>>(codes_in, codes_out, n, vec_ok, scales_in, scales_out,
+                                                                 n_scales, rounded_dev, status_dev, 0, 0);
+  BFP8_CUDA_TRY(cudaGetLastError());
+  return BFP8_OK;
+}
+
+extern "C" int bfp8_reencode_half_swiglu(const uint8_t* codes_in, uint8_t* codes_out, int64_t inter, int64_t k,
+                                         const float* scales_in, float* scales_out, int64_t n_scales,
+                                         unsigned long long* rounded_dev, uint32_t* status_dev, void* stream) {
+  if (!codes_in || !codes_out || !rounded_dev || !status_dev) return BFP8_ERR_NULL;
+  if (inter <= 0 || k <= 0 || inter > (1 << 29) || k > (1 << 30) || n_scales < 0) return BFP8_ERR_SHAPE;
+  if (n_scales > 0 && (!scales_in || !scales_out)) return BFP8_ERR_NULL;
+  if (inter % 128 != 0 || k % 16 != 0) return BFP8_ERR_UNSUPPORTED;
+  if (!aligned(codes_in, 16) || !aligned(codes_out, 16) || !aligned(rounded_dev, 8) || !aligned(status_dev, 4))
+    return BFP8_ERR_ALIGN;
+  if (codes_in == codes_out) return BFP8_ERR_SHAPE;                // not an in-place operation
+  const int64_t vecs = k / 16, total = 2 * inter * vecs;
+  if (total > 0xffffffffLL) return BFP8_ERR_SHAPE;
+  const int64_t per_cta = static_cast<int64_t>(kReencodeThreads) * kReencodeUnroll;            // vectors
+  reencode_half_kernel<true><<<static_cast<int>((total + per_cta - 1) / per_cta), kReencodeThreads, 0,
+                               static_cast<cudaStream_t>(stream)>>>(
+      codes_in, codes_out, total * 16, 1, scales_in, scales_out, n_scales, rounded_dev, status_dev,
+      static_cast<uint32_t>(vecs), static_cast<uint32_t>(inter));
   BFP8_CUDA_TRY(cudaGetLastError());
   return BFP8_OK;
 }

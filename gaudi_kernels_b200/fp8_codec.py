@@ -52,6 +52,16 @@ def reencode_e4m3fn_half(weight, scales):
     codes, `scales` a non-empty contiguous finite non-negative float32 tensor whose doubling must
     not overflow.  The returned bytes are Gaudi2 half-range codes in float8_e4m3fn storage.
     """
+    on_host = isinstance(weight, torch.Tensor) and weight.device.type == "cpu"
+    enc, adj, rounded = _reencode_on_device(weight, scales)
+    if on_host:
+        enc, adj = enc.cpu(), adj.cpu()
+    return enc, adj, rounded
+
+
+def _reencode_on_device(weight, scales, swiglu_inter=0):
+    """reencode_e4m3fn_half with the results left on the device.  swiglu_inter > 0: the weight is a fused gate/up one of
+    2 * swiglu_inter rows (K % 16 == 0) and its codes come back in the row order of gemm_block_fp8_swiglu."""
     if (not isinstance(weight, torch.Tensor) or weight.dtype != torch.float8_e4m3fn
             or not weight.is_contiguous() or not weight.numel() or weight.requires_grad):
         raise ValueError("expected a nonempty contiguous E4M3FN weight")
@@ -60,23 +70,25 @@ def reencode_e4m3fn_half(weight, scales):
         raise ValueError("expected nonempty contiguous finite nonnegative FP32 scales")
     lib = _lib.load()
     dev = _device_for(weight, scales)
-    on_host = weight.device.type == "cpu"
     with torch.cuda.device(dev):
         w = weight.to(dev, non_blocking=True)
         s = scales.to(dev, non_blocking=True)
         enc = torch.empty_like(w)
         adj = torch.empty_like(s)
         st = _status_buffer(dev)
-        rc = lib.bfp8_reencode_half(w.data_ptr(), enc.data_ptr(), w.numel(), s.data_ptr(), adj.data_ptr(),
-                                    s.numel(), st.data_ptr(), st.data_ptr() + 8, _stream_ptr())
-        _lib.check(rc, "bfp8_reencode_half")
+        if swiglu_inter:
+            rc = lib.bfp8_reencode_half_swiglu(w.data_ptr(), enc.data_ptr(), swiglu_inter, w.shape[1], s.data_ptr(),
+                                               adj.data_ptr(), s.numel(), st.data_ptr(), st.data_ptr() + 8, _stream_ptr())
+            _lib.check(rc, "bfp8_reencode_half_swiglu")
+        else:
+            rc = lib.bfp8_reencode_half(w.data_ptr(), enc.data_ptr(), w.numel(), s.data_ptr(), adj.data_ptr(),
+                                        s.numel(), st.data_ptr(), st.data_ptr() + 8, _stream_ptr())
+            _lib.check(rc, "bfp8_reencode_half")
         rounded, status = _read_status(st)
     if status & _lib.STATUS_BAD_SCALE:
         raise ValueError("expected finite nonnegative FP32 scales whose doubling does not overflow FP32")
     if status & _lib.STATUS_NONFINITE_CODE:
         raise ValueError("nonfinite OCP E4M3FN checkpoint code")
-    if on_host:
-        enc, adj = enc.cpu(), adj.cpu()
     return enc, adj, rounded
 
 

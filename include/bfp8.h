@@ -64,6 +64,13 @@ int bfp8_reencode_half(const uint8_t* codes_in, uint8_t* codes_out, int64_t n,
                        const float* scales_in, float* scales_out, int64_t n_scales,
                        unsigned long long* rounded_dev, uint32_t* status_dev, void* stream);
 
+/* bfp8_reencode_half of a fused gate/up weight [2 * inter, k] (contiguous rows) that also puts the codes in the row
+ * order of bfp8_swiglu_interleave_weight: one pass over the weight instead of two, the same bytes.  inter % 128 == 0,
+ * k % 16 == 0, both code buffers 16-byte aligned and distinct, fewer than 2^36 codes. */
+int bfp8_reencode_half_swiglu(const uint8_t* codes_in, uint8_t* codes_out, int64_t inter, int64_t k,
+                              const float* scales_in, float* scales_out, int64_t n_scales,
+                              unsigned long long* rounded_dev, uint32_t* status_dev, void* stream);
+
 /* The input checks of bfp8_reencode_half without the re-encoding, for checkpoints whose OCP codes are used
  * unchanged: status |= NONFINITE_CODE for any 0x7f / 0xff code (python/gaudi_kernels/fp8_codec.py:48-49;
  * python/gaudi_kernels/block_fp8_oracle.py:22-24 rejects the same inputs), BAD_SCALE for a negative or

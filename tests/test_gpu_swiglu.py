@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 import torch
 
-from oracle import block_fp8_ref, swiglu_ref
+from oracle import block_fp8_ref, fp8_codec_ref, swiglu_ref
 
 pytestmark = pytest.mark.gpu
 
@@ -53,6 +53,33 @@ def test_interleave_is_the_documented_row_order(gk, inter, k):
     got, s_out = gk.prepare_weight_swiglu(torch.from_numpy(w).cuda(), torch.from_numpy(s).cuda(), native_half=False)
     assert torch.equal(s_out.cpu(), torch.from_numpy(s))
     assert np.array_equal(got.view(torch.uint8).cpu().numpy()[:, :k], swiglu_ref.interleave_gate_up(w))
+
+
+@pytest.mark.parametrize("inter,k", [(128, 16), (128, 128), (384, 208), (1024, 4096), (128, 1000), (640, 40)])
+def test_prepared_gate_up_equals_reencode_then_interleave(gk, inter, k):
+    # K a multiple of 16 takes the one-pass kernel, the others re-encode and interleave in two; every code occurs
+    rng = np.random.default_rng(inter * 3 + k)
+    w = rng.integers(0, 256, size=(2 * inter, k), dtype=np.uint8)
+    w[(w & 0x7f) == 0x7f] = 0x01
+    s = rng.random((2 * inter // 128, (k + 127) // 128), dtype=np.float32)
+    want, want_s, _ = fp8_codec_ref.reencode_e4m3fn_half(w, s)
+    for device in ("cuda", "cpu"):
+        wt, st = torch.from_numpy(w).view(torch.float8_e4m3fn).to(device), torch.from_numpy(s).to(device)
+        got, got_s = gk.prepare_weight_swiglu(wt, st)
+        assert got.device.type == "cuda" and got.dtype == torch.float8_e4m3fn
+        got = got.view(torch.uint8).cpu().numpy()
+        assert got.shape == (2 * inter, (k + 15) // 16 * 16) and not got[:, k:].any()
+        assert np.array_equal(got[:, :k], swiglu_ref.interleave_gate_up(want))
+        assert np.array_equal(got_s.cpu().numpy(), want_s)
+        assert np.array_equal(wt.view(torch.uint8).cpu().numpy(), w)                   # input untouched
+    bad = w.copy()
+    bad[-1, -1] = 0xff
+    with pytest.raises(ValueError, match="nonfinite"):
+        gk.prepare_weight_swiglu(torch.from_numpy(bad).view(torch.float8_e4m3fn).cuda(), torch.from_numpy(s).cuda())
+    neg = s.copy()
+    neg[-1, -1] = -1.0
+    with pytest.raises(ValueError, match="scales"):
+        gk.prepare_weight_swiglu(torch.from_numpy(w).view(torch.float8_e4m3fn).cuda(), torch.from_numpy(neg).cuda())
 
 
 @pytest.mark.parametrize("m,k,inter,bias", [(1, 128, 128, False), (37, 384, 256, True), (130, 208, 384, False),
