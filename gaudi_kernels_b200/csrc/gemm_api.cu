@@ -28,6 +28,10 @@ int launch_gemm_channel(const uint8_t* a_codes, int64_t lda, const float* a_scal
                         int64_t ldw, const float* w_scales, const float* bias, void* out, int out_dtype, int64_t ldo,
                         int64_t m, int64_t n, int64_t k, uint32_t* status_dev, long long wait_limit, int max_ctas,
                         cudaStream_t st);
+int launch_gemm_smallm_token(const uint8_t* a_codes, int64_t lda, const float* a_scales, const uint8_t* w_codes,
+                             int64_t ldw, const float* w_scales, const float* bias, void* out, int out_dtype,
+                             int64_t ldo, int64_t m, int64_t n, int64_t k, uint32_t* status_dev, long long wait_limit,
+                             cudaStream_t st);
 size_t smallm_workspace_bytes(int64_t m, int64_t n, int max_ctas);
 int set_weights_at_rest(int on);
 bool smallm_supported(int64_t n);
@@ -108,6 +112,11 @@ extern "C" int bfp8_gemm_token_channel(const uint8_t* a_codes, int64_t lda, cons
   if (bias && !aligned(bias, 4)) return BFP8_ERR_ALIGN;
   if (out_dtype == BFP8_OUT_BF16 && (!aligned(out, 16) || ldo % 8 != 0)) return BFP8_ERR_ALIGN;
   if (out_dtype == BFP8_OUT_F32 && !aligned(out, 4)) return BFP8_ERR_ALIGN;
+  // one pass over W: the weight-streaming form (16: 24.3 -> 14.8 us at K=4096, N=14336; 64: 23.6 -> 19.7; at 128 rows its
+  // epilogue paces it and the large tiles are faster, 24.2 against 26.8)
+  if (m <= 64)
+    return launch_gemm_smallm_token(a_codes, lda, a_scales, w_codes, ldw, w_scales, bias, out, out_dtype, ldo, m, n, k,
+                                    status_dev, kDefaultWaitLimit, static_cast<cudaStream_t>(stream));
   return launch_gemm_channel(a_codes, lda, a_scales, w_codes, ldw, w_scales, bias, out, out_dtype, ldo, m, n, k,
                              status_dev, kDefaultWaitLimit, 0, static_cast<cudaStream_t>(stream));
 }

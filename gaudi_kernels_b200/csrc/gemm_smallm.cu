@@ -36,6 +36,12 @@
 // grid (two scale vectors per unit), both factors get their bias and are rounded to bf16 as the unfused GEMM
 // would store them, the up half hands its values to the gate half through shared memory, and the gate half
 // stores bf16(silu(gate) * up) - csrc/tpc/generic_dense/silu_and_mul_bf16.c:16 - into the [M, inter] output.
+//
+// Token form: one fp32 scale per activation row and one per weight row (the per-token / per-channel variant; reference
+// csrc/tpc/block_fp8_framework/channel_finish.c:12-14).  Nothing scales inside the K range, so the units are summed as
+// they are and the result is formed once, (sum * act_scale) * w_scale + bias.  The large-tile kernel gave a decode call
+// 128 x 256 tiles - 56 of 148 SMs at N = 14336, 15/16 of the MMAs on padding rows.  It needs no workspace: a CTA's list is
+// whole tiles, where necessary with tiles beyond N at its end, whose loads are filled with zeros without touching HBM.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -63,6 +69,7 @@ constexpr int kAccBufs = 4;
 constexpr int kWBytes = BN * BK;   // 16 KB of W per unit
 constexpr int kMaxStages = 10;
 constexpr int kSmemBudget = 200 * 1024;
+enum Form { kBlock, kSwiGLUForm, kToken };        // scales per 128 x 128 block, the same with the SwiGLU finish, token form
 constexpr int kSwigluRows = 64;    // activation rows per exchange round of the SwiGLU form (fewer when MP is smaller)
 constexpr int kSwigluExBytes = 2 * kSwigluRows * 64 * 2;   // gate and up values as bf16
 
@@ -175,11 +182,12 @@ __host__ __device__ inline int cta_of_unit(long long u, long long total, long lo
   return static_cast<int>(((u + 1) * parts - 1) / total);
 }
 
-template <int MP, bool kCluster, bool kSwiGLU>
+template <int MP, bool kCluster, Form F>
 __global__ void __launch_bounds__(Cfg<MP>::kThreads, 1)
 gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
                    const Params p) {
   using C = Cfg<MP>;
+  constexpr bool kSwiGLU = F == kSwiGLUForm;
   BFP8_TL_DECL
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -209,7 +217,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     for (int b = 0; b < kAccBufs; ++b) {
       // a buffer is ready for the epilogue when its MMAs have completed (tcgen05.commit) and the scale loader has
       // parked the unit's scale products next to it: two arrivals on one barrier, one poll per unit for the epilogue
-      ptx::mbar_init(ptx::smem_u32(&tail->tmem_full[b]), 2);
+      ptx::mbar_init(ptx::smem_u32(&tail->tmem_full[b]), F == kToken ? 1 : 2);
       ptx::mbar_init(ptx::smem_u32(&tail->tmem_empty[b]), kEpiWarps);
     }
     tail->abort_flag = 0;
@@ -305,6 +313,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
   } else if (warp == kEpiWarps + 2) {
     // ------------------------------------------------------------------ scale loader
+   if (F != kToken) {
     constexpr int kPer = (MP + 31) / 32;                         // activation scales per lane and unit
     // Raw scales of the next kScaleAhead units.  They are multiplied only when their unit comes up: using a
     // loaded value right away would stall this warp for a full L2 round trip on every unit.
@@ -355,6 +364,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         }
       }
     }
+   }
   } else {
     // ------------------------------------------------------------------ epilogue / promotion
     const int wrow = warp * 32 + lane;                         // weight row inside the tile = TMEM lane
@@ -373,6 +383,10 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // thread whose bounded wait expired still calls this for every remaining segment end (alive == false: it takes
     // part in the barriers and the counter protocol, stores nothing), see the loop after the main one.
     long long u = u0;
+    // bias and, in the token form, the scales: what becomes of the sum of activation row j
+    auto result = [&](float sum, int j, float ws, float b) {
+      return F == kToken ? fmaf(sum * __ldg(p.a_scales + j), ws, b) : sum + b;
+    };
     int pending_tile = -1;                                     // tile whose partial is stored but not yet counted in
     // makes this CTA's partial of tile t visible and counts the CTA in at that tile (all 128 epilogue threads)
     auto count_in = [&](int t) {
@@ -446,7 +460,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
           }
         } else if (do_store && alive && col < p.n) {
           const float b = p.bias != nullptr ? __ldg(p.bias + col) : 0.0f;
-          if (p.out_bf16 && p.push_world > 0) {
+          const float ws = F == kToken ? __ldg(p.w_scales + col) : 0.0f;
+          if (F == kBlock && p.out_bf16 && p.push_world > 0) {
 #pragma unroll
             for (int j = 0; j < MP; ++j)
               if (j < p.m) out_row_bf16(p, j)[col] = static_cast<uint16_t>(float_to_bf16_bits(acc[j] + b));
@@ -454,12 +469,12 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             uint16_t* o = reinterpret_cast<uint16_t*>(p.out) + col;
 #pragma unroll
             for (int j = 0; j < MP; ++j)
-              if (j < p.m) o[static_cast<int64_t>(j) * p.ldo] = static_cast<uint16_t>(float_to_bf16_bits(acc[j] + b));
+              if (j < p.m) o[static_cast<int64_t>(j) * p.ldo] = static_cast<uint16_t>(float_to_bf16_bits(result(acc[j], j, ws, b)));
           } else {
             float* o = reinterpret_cast<float*>(p.out) + col;
 #pragma unroll
             for (int j = 0; j < MP; ++j)
-              if (j < p.m) o[static_cast<int64_t>(j) * p.ldo] = acc[j] + b;
+              if (j < p.m) o[static_cast<int64_t>(j) * p.ldo] = result(acc[j], j, ws, b);
           }
         }
 #pragma unroll
@@ -486,6 +501,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         float s[kChunk];
 #pragma unroll
         for (int j = 0; j < kChunk; j += 4) {
+          if (F == kToken) continue;
           const float4 t4 = *reinterpret_cast<const float4*>(&my_scale[buf * 128 + h * kChunk + j]);
           s[j] = t4.x; s[j + 1] = t4.y; s[j + 2] = t4.z; s[j + 3] = t4.w;
         }
@@ -505,7 +521,9 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         for (int c = 0; c < kChunk / 16; ++c)
 #pragma unroll
           for (int j = 0; j < 16; ++j)
-            acc[h * kChunk + c * 16 + j] = fmaf(__uint_as_float(r[c][j]), s[c * 16 + j], acc[h * kChunk + c * 16 + j]);
+            acc[h * kChunk + c * 16 + j] = F == kToken
+                ? acc[h * kChunk + c * 16 + j] + __uint_as_float(r[c][j])
+                : fmaf(__uint_as_float(r[c][j]), s[c * 16 + j], acc[h * kChunk + c * 16 + j]);
       }
       if (!kCluster && (g == G - 1 || u == u1 - 1)) segment_end(true);
     }
@@ -554,6 +572,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         }
       } else if (ok && col < p.n) {
         const float b = p.bias != nullptr ? __ldg(p.bias + col) : 0.0f;
+        const float ws = F == kToken ? __ldg(p.w_scales + col) : 0.0f;
         const float* mine = reinterpret_cast<const float*>(smem);
         // four rows at a time, their sums formed side by side (each is a chain of cs dependent shared-memory loads
         // and adds; one row after the other leaves the thread waiting on every link of every chain)
@@ -568,7 +587,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
           for (int q = 0; q < 4; ++q) {
             const int j = crank * rows_per + jj0 + q;
             if (jj0 + q < rows_per && j < p.m) {
-              const float v = sum[q] + b;
+              const float v = result(sum[q], j, ws, b);
               if (p.out_bf16)
                 out_row_bf16(p, j)[col] = static_cast<uint16_t>(float_to_bf16_bits(v));
               else
@@ -595,12 +614,12 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   if (threadIdx.x == 0 && tail->abort_flag != 0) atomicOr(p.status, BFP8_STATUS_WAIT_TIMEOUT);
 }
 
-template <int MP, bool kSwiGLU>
+template <int MP, Form F>
 int launch(const CUtensorMap& tmap_w, const CUtensorMap& tmap_a, const Params& p, int grid, cudaStream_t st) {
   using C = Cfg<MP>;
-  constexpr int smem = 1024 + C::kStages * C::kStageBytes + sizeof(SmemTail) + (kSwiGLU ? kSwigluExBytes : 0);
+  constexpr int smem = 1024 + C::kStages * C::kStageBytes + sizeof(SmemTail) + (F == kSwiGLUForm ? kSwigluExBytes : 0);
   static DeviceFlags done;
-  const int rc = ensure_smem_limit(gemm_smallm_kernel<MP, false, kSwiGLU>, smem, done);
+  const int rc = ensure_smem_limit(gemm_smallm_kernel<MP, false, F>, smem, done);
   if (rc != BFP8_OK) return rc;
   // launched so that the set-up of this kernel may overlap the tail of the previous kernel in the stream
   cudaLaunchConfig_t cfg = {};
@@ -613,19 +632,19 @@ int launch(const CUtensorMap& tmap_w, const CUtensorMap& tmap_a, const Params& p
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_smallm_kernel<MP, false, kSwiGLU>, tmap_w, tmap_a, p));
+  BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_smallm_kernel<MP, false, F>, tmap_w, tmap_a, p));
   return BFP8_OK;
 }
 
 // Cluster form: p.tiles clusters of p.cluster CTAs.  Returns BFP8_ERR_UNSUPPORTED without launching when the
 // device cannot hold all clusters at once (the caller then uses the plain form).
-template <int MP, bool kSwiGLU>
+template <int MP, Form F>
 int launch_clustered(const CUtensorMap& tmap_w, const CUtensorMap& tmap_a, const Params& p, cudaStream_t st) {
   using C = Cfg<MP>;
-  constexpr int smem = 1024 + C::kStages * C::kStageBytes + sizeof(SmemTail) + (kSwiGLU ? kSwigluExBytes : 0);
+  constexpr int smem = 1024 + C::kStages * C::kStageBytes + sizeof(SmemTail) + (F == kSwiGLUForm ? kSwigluExBytes : 0);
   static_assert(MP * BN * 4 <= C::kStages * C::kStageBytes, "the exchange area reuses the pipeline buffers");
   static DeviceFlags done;
-  const int rc = ensure_smem_limit(gemm_smallm_kernel<MP, true, kSwiGLU>, smem, done);
+  const int rc = ensure_smem_limit(gemm_smallm_kernel<MP, true, F>, smem, done);
   if (rc != BFP8_OK) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(p.tiles * p.cluster), 1, 1);
@@ -648,12 +667,12 @@ int launch_clustered(const CUtensorMap& tmap_w, const CUtensorMap& tmap_a, const
   const int slot = p.cluster == 2 ? 0 : p.cluster == 4 ? 1 : 2;
   int cap = (dev >= 0 && dev < 64) ? max_clusters[dev][slot].load(std::memory_order_acquire) : 0;
   if (cap == 0) {
-    BFP8_CUDA_TRY(cudaOccupancyMaxActiveClusters(&cap, gemm_smallm_kernel<MP, true, kSwiGLU>, &cfg));
+    BFP8_CUDA_TRY(cudaOccupancyMaxActiveClusters(&cap, gemm_smallm_kernel<MP, true, F>, &cfg));
     if (cap <= 0) cap = -1;
     if (dev >= 0 && dev < 64) max_clusters[dev][slot].store(cap, std::memory_order_release);
   }
   if (cap < p.tiles) return BFP8_ERR_UNSUPPORTED;
-  BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_smallm_kernel<MP, true, kSwiGLU>, tmap_w, tmap_a, p));
+  BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_smallm_kernel<MP, true, F>, tmap_w, tmap_a, p));
   return BFP8_OK;
 }
 
@@ -661,24 +680,24 @@ int launch_clustered(const CUtensorMap& tmap_w, const CUtensorMap& tmap_a, const
 
 
 // Cluster form where it applies (and the device can hold all clusters at once), else the plain form.
-template <bool kSwiGLU>
+template <Form F>
 int dispatch(int mp, const CUtensorMap& tmap_w, const CUtensorMap& tmap_a, Params& p, int grid, cudaStream_t st) {
   if (p.cluster >= 2) {
     int crc;
     switch (mp) {
-      case 16: crc = launch_clustered<16, kSwiGLU>(tmap_w, tmap_a, p, st); break;
-      case 32: crc = launch_clustered<32, kSwiGLU>(tmap_w, tmap_a, p, st); break;
-      case 64: crc = launch_clustered<64, kSwiGLU>(tmap_w, tmap_a, p, st); break;
-      default: crc = launch_clustered<128, kSwiGLU>(tmap_w, tmap_a, p, st); break;
+      case 16: crc = launch_clustered<16, F>(tmap_w, tmap_a, p, st); break;
+      case 32: crc = launch_clustered<32, F>(tmap_w, tmap_a, p, st); break;
+      case 64: crc = launch_clustered<64, F>(tmap_w, tmap_a, p, st); break;
+      default: crc = launch_clustered<128, F>(tmap_w, tmap_a, p, st); break;
     }
     if (crc != BFP8_ERR_UNSUPPORTED) return crc;
     p.cluster = 0;
   }
   switch (mp) {
-    case 16: return launch<16, kSwiGLU>(tmap_w, tmap_a, p, grid, st);
-    case 32: return launch<32, kSwiGLU>(tmap_w, tmap_a, p, grid, st);
-    case 64: return launch<64, kSwiGLU>(tmap_w, tmap_a, p, grid, st);
-    default: return launch<128, kSwiGLU>(tmap_w, tmap_a, p, grid, st);
+    case 16: return launch<16, F>(tmap_w, tmap_a, p, grid, st);
+    case 32: return launch<32, F>(tmap_w, tmap_a, p, grid, st);
+    case 64: return launch<64, F>(tmap_w, tmap_a, p, grid, st);
+    default: return launch<128, F>(tmap_w, tmap_a, p, grid, st);
   }
 }
 
@@ -793,8 +812,41 @@ int launch_gemm_smallm(const uint8_t* a_codes, int64_t lda, const float* a_scale
   }
   p.cluster = max_ctas > 0 ? 0 : smallm_cluster_size(p.tiles, p.groups, sms);
   p.w_early = g_weights_at_rest.load(std::memory_order_relaxed);
-  if (inter > 0) return dispatch<true>(mp, tmap_w, tmap_a, p, grid, st);
-  return dispatch<false>(mp, tmap_w, tmap_a, p, grid, st);
+  if (inter > 0) return dispatch<kSwiGLUForm>(mp, tmap_w, tmap_a, p, grid, st);
+  return dispatch<kBlock>(mp, tmap_w, tmap_a, p, grid, st);
+}
+
+// Token form: a_scales fp32 [m], w_scales fp32 [n].
+int launch_gemm_smallm_token(const uint8_t* a_codes, int64_t lda, const float* a_scales, const uint8_t* w_codes,
+                             int64_t ldw, const float* w_scales, const float* bias, void* out, int out_dtype,
+                             int64_t ldo, int64_t m, int64_t n, int64_t k, uint32_t* status_dev, long long wait_limit,
+                             cudaStream_t st) {
+  const int mp = smallm_padded_rows(m);
+  alignas(64) CUtensorMap tmap_w, tmap_a;
+  int rc = make_tensor_map_2d(&tmap_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, w_codes, k, n, ldw, BK, BN);
+  if (rc != BFP8_OK) return rc;
+  rc = make_tensor_map_2d(&tmap_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, a_codes, k, m, lda, BK, mp);
+  if (rc != BFP8_OK) return rc;
+  Params p = {};
+  p.a_scales = a_scales;
+  p.w_scales = w_scales;
+  p.bias = bias;
+  p.out = out;
+  p.ldo = ldo;
+  p.m = static_cast<int>(m);
+  p.n = static_cast<int>(n);
+  p.groups = static_cast<int>((k + BK - 1) / BK);
+  p.tiles = static_cast<int>((n + BN - 1) / BN);
+  p.out_bf16 = out_dtype == BFP8_OUT_BF16;
+  p.wait_limit = wait_limit;
+  p.status = status_dev;
+  p.push_rows = 1;
+  const int sms = sm_count();
+  p.cluster = smallm_cluster_size(p.tiles, p.groups, sms);
+  // every CTA walks the same number of whole tiles (see the file's head): no partial sums, no workspace
+  const int waves = (p.tiles + sms - 1) / sms, grid = (p.tiles + waves - 1) / waves;
+  p.total_units = static_cast<long long>(grid) * waves * p.groups;
+  return dispatch<kToken>(mp, tmap_w, tmap_a, p, grid, st);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -78,6 +78,36 @@ def test_token_channel_gemm_matches_restatement(gk, m, k, n):
             assert bool((num / den <= 0.01).all())          # the reference's device gate, fp8_hybrid_tpcsim_test.cpp:353-379
 
 
+# decode form: clusters of 8, 4 and 2 CTAs per tile, one CTA per tile (more tiles than half the SMs), two tiles per CTA; every
+# padded row count at its edges; fewer K blocks than MMA issuers; K and N that are not multiples of anything.
+# Beyond 128 rows: K slices over clusters of 2, 3 and more CTAs, ragged last slice and columns.
+@pytest.mark.parametrize("m,k,n", [(1, 128, 128), (16, 2048, 640), (17, 1040, 4000), (128, 4096, 6000), (3, 384, 9610),
+                                   (33, 640, 12344), (64, 1000, 19000), (65, 256, 9700), (128, 1152, 19003),
+                                   (129, 4096, 515), (300, 2192, 1032), (513, 5120, 2049)])
+def test_token_channel_gemm_weight_streaming_and_split_forms(gk, m, k, n):
+    g = torch.Generator().manual_seed(m * 5 + n)
+    x = torch.randn((m, k), generator=g).to(torch.bfloat16)
+    w_codes, w_scales = _weights(n, k, seed=m + n)
+    bias = torch.randn(n, generator=g) * 0.1 if m % 2 else None
+    a_codes, a_scales = gk.quantize_act_token(x.cuda(), native_half=True)
+    y64, _ = token_channel_ref.gemm_token_channel(a_codes.view(torch.uint8).cpu().numpy(), a_scales.cpu().numpy(),
+                                                  w_codes, w_scales, None if bias is None else bias.numpy())
+    rms = float(y64.pow(2).mean().sqrt())
+    wc, ws = torch.from_numpy(w_codes).cuda(), torch.from_numpy(w_scales).cuda()
+    outs = []
+    for dtype in (torch.float32, torch.float32, torch.bfloat16):
+        buf = torch.full((m + 2, (n + 7) // 8 * 8 + 8), 0.75, dtype=dtype, device="cuda")
+        out = gk.gemm_token_channel_fp8(a_codes, a_scales, wc, ws, bias=None if bias is None else bias.cuda(),
+                                        out=buf[:m, :n], out_dtype=dtype)
+        assert bool((buf[m:] == 0.75).all()) and bool((buf[:, n:] == 0.75).all())      # nothing written outside
+        outs.append(out.clone())
+    # fp32 sums of k products of E4M3 codes (exact): at most k + 4 roundings of 2^-24 of the largest partial sum, which a
+    # random walk keeps within a few rms; 2e-5 covers K = 5120 in any order of summation
+    assert float((outs[0].double().cpu() - y64).abs().max()) / rms <= 2e-5
+    assert torch.equal(outs[0], outs[1])                                               # fixed summation order
+    assert torch.equal(outs[2], outs[0].to(torch.bfloat16))                            # same accumulator, RNE
+
+
 def test_token_channel_gemm_full_size_linearity(gk):
     # M=8192, K=4096, N=14336 at full size: a seeded row sample against the restatement, and exact linearity in the scales
     m, k, n = 8192, 4096, 14336
