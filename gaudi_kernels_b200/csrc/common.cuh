@@ -258,6 +258,25 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
   return val * u;
 }
 
+// One warp stores a box of 32 rows x 32 fp32 columns, lane l holding row l in v, through 4 KB of shared memory so that
+// every store covers 128 contiguous bytes, whatever the alignment of `out` (element [0][0] of the box) and of its pitch.
+// Stored straight from the registers - one row per lane - each store touches 32 rows: an fp32 result took longer to
+// store than a K = 1000 tile took to compute.  rows / cols: how many of the box exist (may be <= 0 or > 32).
+__device__ __forceinline__ void store_box_f32(float* stage, int lane, const float (&v)[32], float* out, int64_t ldo,
+                                              int rows, int cols) {
+  __syncwarp();                                          // the previous box has been read
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    *reinterpret_cast<float4*>(stage + lane * 32 + ((j ^ (lane & 7)) << 2)) =
+        make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  __syncwarp();
+  if (lane < cols) {
+#pragma unroll 8
+    for (int r = 0; r < 32; ++r)
+      if (r < rows) out[r * ldo + lane] = stage[r * 32 + (((lane >> 2) ^ (r & 7)) << 2) + (lane & 3)];
+  }
+}
+
 // 64 output columns of one row as bf16 with plain stores, only the first `valid` of them.  Used for the
 // last box of a row when N is not a multiple of 8: a bulk tensor store writes whole 16-byte chunks.
 __device__ __forceinline__ void store_row_bf16_guarded(uint16_t* o, const float2* a, int valid) {

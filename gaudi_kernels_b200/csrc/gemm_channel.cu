@@ -254,11 +254,10 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               }
             }
           }
-        } else if (row_ok) {
-          float* o = reinterpret_cast<float*>(p.out) + static_cast<int64_t>(row) * p.ldo + col0 + c * 32;
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (col0 + c * 32 + j < p.n) o[j] = v[j];
+        } else {
+          store_box_f32(reinterpret_cast<float*>(my_stage), lane, v,
+                        reinterpret_cast<float*>(p.out) + static_cast<int64_t>(row0) * p.ldo + col0 + c * 32, p.ldo,
+                        p.m - row0, p.n - (col0 + c * 32));
         }
       }
     }

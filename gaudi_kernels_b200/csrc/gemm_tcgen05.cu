@@ -397,13 +397,14 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           }
         }
       } else {
-        if (row_ok) {
-          float* o = reinterpret_cast<float*>(p.out) + static_cast<int64_t>(row) * p.ldo + col0;
 #pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            if (col0 + 2 * j < p.n) o[2 * j] = acc[j].x;
-            if (col0 + 2 * j + 1 < p.n) o[2 * j + 1] = acc[j].y;
-          }
+        for (int b = 0; b < 4; ++b) {
+          float v[32];
+#pragma unroll
+          for (int j = 0; j < 16; ++j) { v[2 * j] = acc[b * 16 + j].x; v[2 * j + 1] = acc[b * 16 + j].y; }
+          const int row0 = tm * BM + quad * 32, c = col0 + b * 32;
+          store_box_f32(reinterpret_cast<float*>(my_stage), lane, v,
+                        reinterpret_cast<float*>(p.out) + static_cast<int64_t>(row0) * p.ldo + c, p.ldo, p.m - row0, p.n - c);
         }
       }
     }

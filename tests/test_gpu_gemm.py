@@ -184,6 +184,25 @@ def test_gemm_small_m_cluster_exchange(gk, m, k, n):
     assert torch.equal(out16, out.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("m,n,ldo", [(129, 1, 1), (130, 257, 257), (200, 1003, 1003), (300, 384, 390), (1030, 250, 251)])
+def test_gemm_fp32_result_any_pitch(gk, m, n, ldo):
+    # fp32 rows of any pitch and alignment: boxes of 32 x 32 are stored through shared memory
+    k = 256
+    x, w, s, b = _random_problem(m, k, n, seed=n, bias=True)
+    a_codes, a_scales = gk.quantize_act_1x128(x.cuda(), native_half=True)
+    wc, ws = gk.prepare_weight(w, s, native_half=True)
+    y64, _ = block_fp8_ref.reference_rows(x, w, s, native_half=True, bias=b)
+    rms = float(y64.pow(2).mean().sqrt())
+    flat = torch.full((1 + (m + 1) * ldo,), 0.5, device="cuda")             # starts 4 bytes past a 16-byte boundary
+    out = flat[1:1 + m * ldo].view(m, ldo)[:, :n]
+    gk.gemm_block_fp8(a_codes, a_scales, wc, ws, bias=b.cuda(), out=out, out_dtype=torch.float32, schedule=1)
+    assert float((out.double().cpu() - y64).abs().max()) / rms <= TOL
+    rest = flat[1:].view(m + 1, ldo)
+    assert bool((rest[m:] == 0.5).all()) and bool((rest[:, n:] == 0.5).all()) and float(flat[0]) == 0.5
+    out16 = gk.gemm_block_fp8(a_codes, a_scales, wc, ws, bias=b.cuda(), schedule=1)
+    assert torch.equal(out16, out.to(torch.bfloat16))
+
+
 def test_gemm_output_tail_is_untouched(gk):
     # sentinel columns right of N and rows below M must survive (out-of-bounds write check)
     m, k, n = 70, 256, 203
