@@ -64,6 +64,13 @@ def _group_major(a_scales, m, g):
     return t, m
 
 
+def _row_independent_schedule(m):
+    """The schedule whose result bits do not depend on how many rows or columns the call covers: beyond the decode
+    bucket the automatic schedule may sum a tile's K range in slices, the large-tile schedule adds K blocks in order.
+    For callers whose contract is that a row block, a column shard or a fused exchange gives the same bits."""
+    return 1 if m > 128 else 0
+
+
 def wait_timed_out(status):
     """True if a kernel given `status` (a tensor from new_status()) reported an expired bounded wait.
 
@@ -99,6 +106,9 @@ def gemm_block_fp8(a_codes, a_scales, w_codes, w_scales, bias=None, out=None, ou
     a_scales fp32 [M, G]; group-major storage (as returned by quantize_act_1x128) avoids a copy
     w_codes  E4M3 [N, K], contiguous;  w_scales fp32 [ceil(N/128), G] contiguous
     bias     fp32 [N] or None;  out_dtype torch.bfloat16 (default) or torch.float32
+    schedule 0 (default) chooses by size: weight streaming for M <= 128; beyond that 128 x 256 tiles, whose K range is
+             summed in slices by several SMs where there are too few tiles to occupy the GPU.  1 large tiles with
+             K blocks added in order, 2 weight streaming, 3 CTA pairs
     check    read the device status word after the launch (one synchronisation) and raise if a
              bounded wait expired; pass False on a latency-critical path together with `status`
     status   a buffer from new_status() that receives the kernel's status bits; several calls may share one.
@@ -381,7 +391,7 @@ def reference(x, weight, scales, *, native_half=False, bias=None, out_dtype=torc
                                                st.data_ptr() + 8, _stream_ptr())
             _lib.check(rc, "bfp8_quant_act_1x128_bf16")
             return gemm_block_fp8(a_codes, a_scales.t(), enc, sw, bias=bias, out=dev_out, out_dtype=out_dtype,
-                                  check=False, status=st)
+                                  check=False, status=st, schedule=_row_independent_schedule(mr))
 
         if not on_host:
             dev_out = out if (out is not None and out.device.type == "cuda") else None

@@ -86,6 +86,25 @@ inline int ensure_smem_limit(Kernel kernel, int bytes, DeviceFlags& done) {
   return BFP8_OK;
 }
 
+// Clusters of a kernel the current device can hold at once (0 on error), asked once per device and cluster size.  The
+// kernel's shared-memory limit has to be raised first and `cfg` must carry the cluster dimension.
+typedef std::atomic<int> ClusterCaps[64][9];
+template <typename Kernel>
+inline int max_active_clusters(Kernel kernel, const cudaLaunchConfig_t& cfg, int cluster, ClusterCaps& caps) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cluster < 1 || cluster > 8) return 0;
+  const bool slot = dev >= 0 && dev < 64;
+  int cap = slot ? caps[dev][cluster].load(std::memory_order_acquire) : 0;
+  if (cap == 0) {
+    if (cudaOccupancyMaxActiveClusters(&cap, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();                            // not left behind for the caller's next check
+      cap = 0;
+    }
+    if (slot) caps[dev][cluster].store(cap > 0 ? cap : -1, std::memory_order_release);
+  }
+  return cap > 0 ? cap : 0;
+}
+
 // Launch with the programmatic-stream-serialization attribute: the kernel may be scheduled while the previous
 // kernel of the stream is still finishing and must call ptx::griddep_wait() (or the griddepcontrol.wait
 // instruction) before it touches global memory.  Used for the short kernels of a decode step, where the launch

@@ -13,7 +13,7 @@ struct SmallPush {
 int launch_gemm_large(const uint8_t* a_codes, int64_t lda, const float* a_scales, int64_t ldsa,
                       const uint8_t* w_codes, int64_t ldw, const float* w_scales, const float* bias, void* out,
                       int out_dtype, int64_t ldo, int64_t m, int64_t n, int64_t k, uint32_t* status_dev,
-                      long long wait_limit, int max_ctas, int band, int inter, const PushTarget* push,
+                      long long wait_limit, int max_ctas, int band, int inter, const PushTarget* push, bool may_split,
                       cudaStream_t st);
 int launch_gemm_pair(const uint8_t* a_codes, int64_t lda, const float* a_scales, int64_t ldsa,
                      const uint8_t* w_codes, int64_t ldw, const float* w_scales, const float* bias, void* out,
@@ -85,7 +85,7 @@ extern "C" int bfp8_gemm_block128_ex(const uint8_t* a_codes, int64_t lda, const 
     return launch_gemm_pair(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, bias, out, out_dtype, ldo, m, n, k,
                             status_dev, limit, max_ctas, st);
   return launch_gemm_large(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, bias, out, out_dtype, ldo, m, n, k,
-                           status_dev, limit, max_ctas, /*band=*/0, /*inter=*/0, /*push=*/nullptr, st);
+                           status_dev, limit, max_ctas, /*band=*/0, /*inter=*/0, /*push=*/nullptr, /*may_split=*/schedule == 0, st);
 }
 
 extern "C" int bfp8_gemm_block128(const uint8_t* a_codes, int64_t lda, const float* a_scales, int64_t ldsa,
@@ -184,7 +184,7 @@ extern "C" int bfp8_gemm_block128_swiglu(const uint8_t* a_codes, int64_t lda, co
   }
   return launch_gemm_large(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, bias, out, BFP8_OUT_BF16, ldo,
                            m, 2 * inter, k, status_dev, kDefaultWaitLimit, 0, /*band=*/0, static_cast<int>(inter),
-                           /*push=*/nullptr, static_cast<cudaStream_t>(stream));
+                           /*push=*/nullptr, /*may_split=*/false, static_cast<cudaStream_t>(stream));
 }
 
 // ---- the SwiGLU step on its own, for results of the schedules that have no fused form (decode bucket) -------
@@ -277,5 +277,5 @@ extern "C" int bfp8_gemm_block128_push(const uint8_t* a_codes, int64_t lda, cons
   }
   return launch_gemm_large(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, nullptr, const_cast<void*>(t.recv[rank]),
                            BFP8_OUT_BF16, n, m, n, k, status_dev, kDefaultWaitLimit, 0, /*band=*/0, /*inter=*/0, &t,
-                           static_cast<cudaStream_t>(stream));
+                           /*may_split=*/false, static_cast<cudaStream_t>(stream));
 }

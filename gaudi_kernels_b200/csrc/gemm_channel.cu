@@ -17,9 +17,11 @@
 
 #include "common.cuh"
 #include "ptx.cuh"
+#include "split_exchange.cuh"
 
 namespace bfp8 {
 
+int split_cluster_size(int64_t tiles, int64_t groups, int sms);
 
 namespace {
 
@@ -55,6 +57,7 @@ struct Params {
   int64_t ldo;
   int m, n, groups;
   int tiles_m, tiles_n;
+  int split;               // CTAs (one cluster) that share a tile's K range in the split form, else 1
   long long wait_limit;
   uint32_t* status;
 };
@@ -70,7 +73,9 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   tn = r / rows;
 }
 
-template <bool kOutBf16>
+// kSplit: few tiles and a long K range, so p.split CTAs form a cluster, each accumulates an equal slice of the tile's K
+// blocks and the partial tiles are exchanged and added as split_exchange.cuh describes.  One tile per cluster.
+template <bool kOutBf16, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                     const __grid_constant__ CUtensorMap tmap_out, const Params p) {
@@ -84,7 +89,13 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int num_tiles = p.tiles_m * p.tiles_n;
-  const int G = p.groups;
+  // this CTA's first tile, the distance to its next, and its K blocks [g_first, g_first + G) of each
+  const int cs = kSplit ? p.split : 1;
+  const int crank = kSplit ? static_cast<int>(blockIdx.x % cs) : 0;
+  const int tile0 = kSplit ? static_cast<int>(blockIdx.x / cs) : static_cast<int>(blockIdx.x);
+  const int tile_step = kSplit ? num_tiles : static_cast<int>(gridDim.x);
+  const int g_first = kSplit ? static_cast<int>(static_cast<long long>(crank) * p.groups / cs) : 0;
+  const int G = kSplit ? static_cast<int>(static_cast<long long>(crank + 1) * p.groups / cs) - g_first : p.groups;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -111,6 +122,9 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
+  // the set-up above touches no global memory and may overlap the previous kernel of the stream
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
 
   if (warp >= kEpiWarps) {
     ptx::setmaxnreg_dec<40>();
@@ -119,7 +133,7 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       if (lane == 0) {
         uint32_t stage = 0, phase = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+        for (int t = tile0; t < num_tiles && ok; t += tile_step) {
           int tm, tn;
           tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
           for (int g = 0; g < G; ++g) {
@@ -128,8 +142,8 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             const uint32_t full = ptx::smem_u32(&tail->full[stage]);
             const uint32_t a_dst = smem_base + stage * kStageBytes;
             ptx::mbar_arrive_expect_tx(full, kStageBytes);
-            ptx::tma_load_2d(a_dst, &tmap_a, full, g * BK, tm * BM);
-            ptx::tma_load_2d(a_dst + kABytes, &tmap_w, full, g * BK, tn * BN);
+            ptx::tma_load_2d(a_dst, &tmap_a, full, (g_first + g) * BK, tm * BM);
+            ptx::tma_load_2d(a_dst + kABytes, &tmap_w, full, (g_first + g) * BK, tn * BN);
             if (++stage == kStages) { stage = 0; phase ^= 1u; }
           }
         }
@@ -140,7 +154,7 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         constexpr uint32_t idesc = ptx::umma_idesc_e4m3(BM, BN);
         uint32_t stage = 0, phase = 0, it = 0;
         bool ok = true;
-        for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
+        for (int t = tile0; t < num_tiles && ok; t += tile_step, ++it) {
           const uint32_t buf = it & 1u, acc_phase = (it >> 1) & 1u;
           ok = ptx::mbar_wait(ptx::smem_u32(&tail->tmem_empty[buf]), acc_phase ^ 1u, abort_flag, p.wait_limit);
           if (!ok) break;
@@ -173,7 +187,7 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint8_t* my_stage = out_stage + warp * kOutWarpBytes;
     uint32_t it = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
+    for (int t = tile0; t < num_tiles && ok; t += tile_step, ++it) {
       int tm, tn;
       tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
       const int row0 = tm * BM + quad * 32;
@@ -187,6 +201,30 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       if (!ok) break;
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + lane_addr + buf * BN + wg * 128;
+      if (kSplit) {
+        ptx::cluster_sync_all();                       // every CTA's pipeline buffers are idle
+        const int trow = quad * 32 + lane;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[32];
+          ptx::tmem_ld32(taddr + c * 32, r);
+          ptx::tmem_wait_ld32(r);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[8 * u + j]);
+            split::send(smem_base, cs, crank, wg * 16 + c * 4 + u, trow, v);
+          }
+        }
+        ptx::cluster_sync_all();                       // every partial sum has arrived
+        split::finish<kOutBf16>(smem, cs, crank, threadIdx.x, kEpiWarps * 32, p.out, p.ldo, tm * BM, tn * BN, p.m, p.n,
+                                [&](int r, int c, float x) {
+                                  return fmaf(x * __ldg(p.a_scales + r), __ldg(p.w_scales + c),
+                                              p.bias != nullptr ? __ldg(p.bias + c) : 0.0f);
+                                });
+        continue;
+      }
       uint32_t ra[32], rb[32];
       ptx::tmem_ld32(taddr, ra);
       ptx::tmem_ld32(taddr + 32, rb);
@@ -261,7 +299,18 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
       }
     }
-    if (kOutBf16 && lane == 0) ptx::tma_store_wait_all();
+    if (kSplit && !ok) {
+      // gave up inside the slice: keep the two appointments of the exchange
+      ptx::cluster_sync_all();
+      ptx::cluster_sync_all();
+    }
+    if (kOutBf16 && !kSplit && lane == 0) ptx::tma_store_wait_all();
+  }
+  if (kSplit && warp >= kEpiWarps) {
+    // the other roles take part in the two cluster barriers of the exchange
+    __syncwarp();
+    ptx::cluster_sync_all();
+    ptx::cluster_sync_all();
   }
 
   // ------------------------------------------------------------------ teardown
@@ -308,12 +357,43 @@ int launch_gemm_channel(const uint8_t* a_codes, int64_t lda, const float* a_scal
   int grid = sm_count();
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (tiles < grid) grid = tiles;
-  auto kern = bf16 ? gemm_channel_kernel<true> : gemm_channel_kernel<false>;
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  p.split = 1;
+  const int want = max_ctas <= 0 ? split_cluster_size(tiles, p.groups, sm_count()) : 1;
+  if (want > 1) {
+    auto kern = bf16 ? gemm_channel_kernel<true, true> : gemm_channel_kernel<false, true>;
+    static DeviceFlags done[2];
+    rc = ensure_smem_limit(kern, kSmemBytes, done[bf16 ? 1 : 0]);
+    if (rc != BFP8_OK) return rc;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+    static ClusterCaps caps;
+    for (int cs = want; cs > 1; --cs) {                // the largest cluster of which the device holds all `tiles` at once
+      attr[1].val.clusterDim.x = static_cast<unsigned>(cs);
+      cfg.gridDim = dim3(static_cast<unsigned>(tiles * cs), 1, 1);
+      if (max_active_clusters(kern, cfg, cs, caps) < tiles) continue;
+      p.split = cs;
+      BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmap_a, tmap_w, tmap_out, p));
+      return BFP8_OK;
+    }
+    cfg.numAttrs = 1;
+  }
+  auto kern = bf16 ? gemm_channel_kernel<true, false> : gemm_channel_kernel<false, false>;
   static DeviceFlags done[2];
   rc = ensure_smem_limit(kern, kSmemBytes, done[bf16 ? 1 : 0]);
   if (rc != BFP8_OK) return rc;
-  kern<<<grid, kThreads, kSmemBytes, st>>>(tmap_a, tmap_w, tmap_out, p);
-  BFP8_CUDA_TRY(cudaGetLastError());
+  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmap_a, tmap_w, tmap_out, p));
   return BFP8_OK;
 }
 

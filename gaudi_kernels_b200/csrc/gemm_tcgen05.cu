@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "ptx.cuh"
+#include "split_exchange.cuh"
 
 namespace bfp8 {
 
@@ -78,6 +79,7 @@ struct GemmParams {
   // Push mode (row-parallel GEMM): the bf16 tile of rows [o R, (o + 1) R) goes to GPU o, into slot `push_rank` of
   // its receive area [push_world][R][N]; push_world == 0 stores to `out` as usual
   int push_world, push_rank, push_rows;
+  int split;               // CTAs (one cluster) that share a tile's K range in the split form, else 1
   int band_shift;          // the tile walk starts at this band (all bands full), so that ranks push to different owners
   long long wait_limit;
   uint32_t* status;
@@ -106,7 +108,10 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
 // tile columns of a warpgroup are 64 gate columns followed by the 64 up columns of the same outputs, and a
 // thread ends a tile holding both factors of its 64 outputs.  The tile's 256 weight rows are outputs
 // 128 tn .. 128 tn + 127, which lie in one scale block of the gate grid and one of the up grid.
-template <bool kOutBf16, bool kSwiGLU>
+// kSplit: few tiles and a long K range would leave most SMs idle, so p.split CTAs form a cluster, each sums an equal
+// slice of the tile's K blocks and the partial tiles are exchanged and added as split_exchange.cuh describes.  One tile
+// per cluster.
+template <bool kOutBf16, bool kSwiGLU, bool kSplit = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                      const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ PushMaps pmaps,
@@ -122,7 +127,13 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int num_tiles = p.tiles_m * p.tiles_n;
-  const int G = p.groups;
+  // this CTA's first tile, the distance to its next, and its K blocks [g_first, g_first + G) of each
+  const int cs = kSplit ? p.split : 1;
+  const int crank = kSplit ? static_cast<int>(blockIdx.x % cs) : 0;
+  const int tile0 = kSplit ? static_cast<int>(blockIdx.x / cs) : static_cast<int>(blockIdx.x);
+  const int tile_step = kSplit ? num_tiles : static_cast<int>(gridDim.x);
+  const int g_first = kSplit ? static_cast<int>(static_cast<long long>(crank) * p.groups / cs) : 0;
+  const int G = kSplit ? static_cast<int>(static_cast<long long>(crank + 1) * p.groups / cs) - g_first : p.groups;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -145,6 +156,9 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
+  // the set-up above touches no global memory and may overlap the previous kernel of the stream
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
 
   if (warp >= kEpiWarps) {
    ptx::setmaxnreg_dec<24>();
@@ -154,7 +168,7 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       uint32_t stage = 0, phase = 0;
       long long pkb = 0;                                        // running K block number (timeline build only)
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      for (int t = tile0; t < num_tiles && ok; t += tile_step) {
         int tm, tn;
         tile_coords(t, p.tiles_m, p.tiles_n, p.band, p.band_shift, tm, tn);
         for (int g = 0; g < G; ++g) {
@@ -165,8 +179,8 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           const uint32_t full = ptx::smem_u32(&tail->full[stage]);
           const uint32_t a_dst = smem_base + stage * kStageBytes;
           ptx::mbar_arrive_expect_tx(full, kStageBytes);
-          ptx::tma_load_2d(a_dst, &tmap_a, full, g * BK, tm * BM);
-          ptx::tma_load_2d(a_dst + kABytes, &tmap_w, full, g * BK, tn * BN);
+          ptx::tma_load_2d(a_dst, &tmap_a, full, (g_first + g) * BK, tm * BM);
+          ptx::tma_load_2d(a_dst + kABytes, &tmap_w, full, (g_first + g) * BK, tn * BN);
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
@@ -178,7 +192,7 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       const uint32_t parity = warp - (kEpiWarps + 1);          // which K blocks, and which TMEM buffer, are mine
       const uint32_t d = tmem_base + parity * BN;
       long long total = 0;                                     // K blocks of this CTA
-      for (int t = blockIdx.x; t < num_tiles; t += gridDim.x) total += G;
+      for (int t = tile0; t < num_tiles; t += tile_step) total += G;
       for (long long kb = parity; kb < total; kb += 2) {
         const uint32_t stage = static_cast<uint32_t>(kb) & (kStages - 1), phase = static_cast<uint32_t>(kb >> 2) & 1u;
         if (!ptx::mbar_wait(ptx::smem_u32(&tail->full[stage]), phase, abort_flag, p.wait_limit)) break;
@@ -212,7 +226,7 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       ptx::mbar_arrive(ptx::smem_u32(&tail->full[0]));
       ptx::mbar_arrive(ptx::smem_u32(&tail->full[1]));
     }
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+    for (int t = tile0; t < num_tiles && ok; t += tile_step) {
       int tm, tn;
       tile_coords(t, p.tiles_m, p.tiles_n, p.band, p.band_shift, tm, tn);
       const int row = tm * BM + quad * 32 + lane;
@@ -221,10 +235,10 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       const bool row_ok = row < p.m;
       const int nb = kSwiGLU ? tn : col0 >> 7;
       const bool live = row_ok && (kSwiGLU || col0 < p.n);
-      const float* sa_ptr = p.a_scales + row;
-      const float* sw_ptr = p.w_scales + static_cast<int64_t>(nb) * G;
+      const float* sa_ptr = p.a_scales + static_cast<int64_t>(g_first) * p.ldsa + row;
+      const float* sw_ptr = p.w_scales + static_cast<int64_t>(nb) * p.groups + g_first;
       // SwiGLU: scale row of the up projection's block (the grid lists the gate blocks first)
-      const float* su_ptr = p.w_scales + static_cast<int64_t>((p.inter >> 7) + nb) * G;
+      const float* su_ptr = p.w_scales + static_cast<int64_t>((p.inter >> 7) + nb) * p.groups;
       float2 acc[64];
 #pragma unroll
       for (int j = 0; j < 64; ++j) acc[j] = make_float2(0.0f, 0.0f);
@@ -310,6 +324,21 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         if (kSwiGLU) { su0 = su1; su1 = su2; }
       }
       if (!ok) break;
+      if (kSplit) {
+        // ---- slice done: exchange the partial tiles, finish this CTA's columns of the sum
+        ptx::cluster_sync_all();                       // every CTA's pipeline buffers are idle
+        const int trow = quad * 32 + lane;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+          const float v[8] = {acc[4 * u].x,     acc[4 * u].y,     acc[4 * u + 1].x, acc[4 * u + 1].y,
+                              acc[4 * u + 2].x, acc[4 * u + 2].y, acc[4 * u + 3].x, acc[4 * u + 3].y};
+          split::send(smem_base, cs, crank, wg * 16 + u, trow, v);
+        }
+        ptx::cluster_sync_all();                       // every partial sum has arrived
+        split::finish<kOutBf16>(smem, cs, crank, threadIdx.x, kEpiWarps * 32, p.out, p.ldo, tm * BM, tn * BN, p.m, p.n,
+                                [&](int, int c, float x) { return p.bias != nullptr ? x + __ldg(p.bias + c) : x; });
+        continue;
+      }
       // ---- tile done: bias, rounding, store
       if (kSwiGLU) {
         // gate and up are rounded to bf16 as the unfused GEMM would store them, then silu(gate) * up is
@@ -408,7 +437,18 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         }
       }
     }
-    if (kOutBf16 && lane == 0) ptx::tma_store_wait_all();
+    if (kSplit && !ok) {
+      // gave up inside the slice: keep the two appointments of the exchange
+      ptx::cluster_sync_all();
+      ptx::cluster_sync_all();
+    }
+    if (kOutBf16 && !kSplit && lane == 0) ptx::tma_store_wait_all();
+  }
+  if (kSplit && warp >= kEpiWarps) {
+    // the other roles take part in the two cluster barriers of the exchange
+    __syncwarp();
+    ptx::cluster_sync_all();
+    ptx::cluster_sync_all();
   }
 
   // ------------------------------------------------------------------ teardown
@@ -466,11 +506,29 @@ int make_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* bas
   return BFP8_OK;
 }
 
+// CTAs per tile of the split form (1: no split), priced with what B200 measured: a K block takes 0.48 us, a launch that
+// splits pays 1.0 us and 1.2 us per CTA of the cluster on top (two cluster barriers, the sends, the columns' sums; 7.9
+// against 9.2 us at M=300, K=N=1024 with two CTAs, 11.1 / 11.4 us at K=N=2048 with four, 18.0 / 14.6 us at M=200, K=4096,
+// N=2048 with eight).  Never more CTAs than the SMs hold at once, a portable cluster, or the K blocks there are.
+int split_cluster_size(int64_t tiles, int64_t groups, int sms) {
+  int64_t most = sms / tiles;
+  if (most > split::kMaxCluster) most = split::kMaxCluster;
+  if (most > groups) most = groups;
+  int best = 1;
+  int64_t best_cost = groups * 48;                       // 0.01 us
+  for (int64_t cs = 2; cs <= most; ++cs) {
+    const int64_t cost = (groups + cs - 1) / cs * 48 + 100 + 120 * cs;
+    if (cost < best_cost) { best_cost = cost; best = static_cast<int>(cs); }
+  }
+  return best;
+}
+
 int launch_gemm_large(const uint8_t* a_codes, int64_t lda, const float* a_scales, int64_t ldsa,
                       const uint8_t* w_codes, int64_t ldw, const float* w_scales, const float* bias, void* out,
                       int out_dtype, int64_t ldo, int64_t m, int64_t n, int64_t k, uint32_t* status_dev,
-                      long long wait_limit, int max_ctas, int band, int inter, const PushTarget* push,
+                      long long wait_limit, int max_ctas, int band, int inter, const PushTarget* push, bool may_split,
                       cudaStream_t st) {
+  // may_split: the caller accepts sums formed in slices of K (schedule 0); otherwise K blocks are added in order
   // inter > 0 selects the SwiGLU epilogue: W has n = 2 * inter interleaved rows and the output is [m, inter] bf16
   // push != nullptr selects the push mode: bf16 tiles go to the receive areas of the GPUs that own their rows
   alignas(64) CUtensorMap tmap_a, tmap_w, tmap_out;
@@ -531,13 +589,44 @@ int launch_gemm_large(const uint8_t* a_codes, int64_t lda, const float* a_scales
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (tiles < grid) grid = tiles;
   if (inter > 0 && !bf16) return BFP8_ERR_UNSUPPORTED;
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  p.split = 1;
+  const int want = (may_split && inter == 0 && push == nullptr && max_ctas <= 0) ? split_cluster_size(tiles, p.groups, sm_count()) : 1;
+  if (want > 1) {
+    auto kern = bf16 ? gemm_block128_kernel<true, false, true> : gemm_block128_kernel<false, false, true>;
+    static DeviceFlags done[2];
+    rc = ensure_smem_limit(kern, kSmemBytes, done[bf16 ? 1 : 0]);
+    if (rc != BFP8_OK) return rc;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+    static ClusterCaps caps;
+    for (int cs = want; cs > 1; --cs) {                // the largest cluster of which the device holds all `tiles` at once
+      attr[1].val.clusterDim.x = static_cast<unsigned>(cs);
+      cfg.gridDim = dim3(static_cast<unsigned>(tiles * cs), 1, 1);
+      if (max_active_clusters(kern, cfg, cs, caps) < tiles) continue;
+      p.split = cs;
+      BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmap_a, tmap_w, tmap_out, pmaps, p));
+      return BFP8_OK;
+    }
+    cfg.numAttrs = 1;
+  }
   auto kern = inter > 0 ? gemm_block128_kernel<true, true>
                         : (bf16 ? gemm_block128_kernel<true, false> : gemm_block128_kernel<false, false>);
   static DeviceFlags done[3];
   rc = ensure_smem_limit(kern, kSmemBytes, done[inter > 0 ? 2 : (bf16 ? 1 : 0)]);
   if (rc != BFP8_OK) return rc;
-  kern<<<grid, kThreads, kSmemBytes, st>>>(tmap_a, tmap_w, tmap_out, pmaps, p);
-  BFP8_CUDA_TRY(cudaGetLastError());
+  cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmap_a, tmap_w, tmap_out, pmaps, p));
   return BFP8_OK;
 }
 

@@ -203,7 +203,7 @@ def gemm_k_sharded(a_codes_local, a_scales_local, w_codes_local, w_scales_local,
     Either form reports an expired bounded wait (GEMM or barrier) through exchange.timed_out().
     fused=None picks the fused form where it applies.
     """
-    from .block_fp8_gemm import _group_major, _workspace, gemm_block_fp8
+    from .block_fp8_gemm import _group_major, _row_independent_schedule, _workspace, gemm_block_fp8
     m, k = a_codes_local.shape
     n = w_codes_local.shape[0]
     world, rank = exchange.world, exchange.rank
@@ -216,7 +216,8 @@ def gemm_k_sharded(a_codes_local, a_scales_local, w_codes_local, w_scales_local,
     if not fused:
         partial = exchange.partial(m, n, partial_dtype)
         gemm_block_fp8(a_codes_local, a_scales_local, w_codes_local, w_scales_local, out=partial,
-                       out_dtype=partial_dtype, check=False, status=exchange.status)
+                       out_dtype=partial_dtype, check=False, status=exchange.status,
+                       schedule=_row_independent_schedule(m))       # the bits of the fused form
         return reduce_scatter_rows(exchange, partial, bias=bias, out=out)
 
     rows = m // world

@@ -88,7 +88,8 @@ def reference_sharded(x_local, weight_local, scales_local, *, native_half=True, 
     it contains two all-gathers and one small all-reduce of the status bits.
     """
     from . import _lib
-    from .block_fp8_gemm import _copy_stream, _workspaces, _WAIT_TIMEOUT_MSG, gemm_block_fp8
+    from .block_fp8_gemm import (_copy_stream, _row_independent_schedule, _workspaces, _WAIT_TIMEOUT_MSG,
+                                 gemm_block_fp8)
     from .fp8_codec import _device_for, _status_buffer, _stream_ptr
     if (x_local.dtype != torch.bfloat16 or weight_local.dtype != torch.float8_e4m3fn or scales_local.dtype != torch.float32
             or x_local.ndim != 2 or weight_local.ndim != 2 or x_local.shape[1] != weight_local.shape[1]):
@@ -126,7 +127,8 @@ def reference_sharded(x_local, weight_local, scales_local, *, native_half=True, 
         a_codes, a_scales = gather_quantized_rows(codes_local, scales_l, group)
         if not on_host:
             y = gemm_block_fp8(a_codes, a_scales.t(), enc, sw, bias=bias_local,
-                               out=out if (out is not None and out.device.type == "cuda") else None, check=False, status=st)
+                               out=out if (out is not None and out.device.type == "cuda") else None, check=False, status=st,
+                               schedule=_row_independent_schedule(m))
         else:
             if out is None:
                 out = torch.empty((m, n_local), dtype=torch.bfloat16)
@@ -140,7 +142,8 @@ def reference_sharded(x_local, weight_local, scales_local, *, native_half=True, 
             keep = []
             for r0 in range(0, m, per):
                 r1 = min(m, r0 + per)
-                yr = gemm_block_fp8(a_codes[r0:r1], a_scales[:, r0:r1].t(), enc, sw, bias=bias_local, check=False, status=st)
+                yr = gemm_block_fp8(a_codes[r0:r1], a_scales[:, r0:r1].t(), enc, sw, bias=bias_local, check=False, status=st,
+                                    schedule=_row_independent_schedule(r1 - r0))
                 done = torch.cuda.Event()
                 done.record(main)
                 side.wait_event(done)

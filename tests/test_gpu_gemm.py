@@ -184,6 +184,32 @@ def test_gemm_small_m_cluster_exchange(gk, m, k, n):
     assert torch.equal(out16, out.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("m,k,n", [(129, 4096, 255), (200, 2176, 1003), (256, 14336, 512), (300, 4096, 4096), (300, 2048, 2048),
+                                   (513, 3000, 1032), (640, 6144, 2816)])
+def test_gemm_split_k_matches_ordered_sum(gk, m, k, n):
+    # too few tiles for the GPU: clusters of 2 to 8 CTAs (these shapes reach 2, 3, 4, 5 and 6) sum slices of a tile's K range;
+    # ragged rows, columns and last K block
+    x, w, s, b = _random_problem(m, k, n, seed=m + k + n, bias=(m % 2 == 0))
+    a_codes, a_scales = gk.quantize_act_1x128(x.cuda(), native_half=True)
+    wc, ws = gk.prepare_weight(w, s, native_half=True)
+    bd = None if b is None else b.cuda()
+    rows = torch.linspace(0, m - 1, 40).long()
+    y64, _ = block_fp8_ref.reference_rows(x[rows], w, s, native_half=True, bias=b)
+    rms = float(y64.pow(2).mean().sqrt())
+    outs = []
+    for dtype, schedule in ((torch.float32, 0), (torch.float32, 0), (torch.bfloat16, 0), (torch.float32, 1)):
+        buf = torch.full((m + 2, (n + 7) // 8 * 8 + 8), 0.75, dtype=dtype, device="cuda")
+        out = gk.gemm_block_fp8(a_codes, a_scales, wc, ws, bias=bd, out=buf[:m, :n], out_dtype=dtype, schedule=schedule)
+        assert bool((buf[m:] == 0.75).all()) and bool((buf[:, n:] == 0.75).all())      # nothing written outside
+        outs.append(out.clone())
+    split, again, half, ordered = outs
+    assert torch.equal(split, again)                                       # fixed summation order
+    assert torch.equal(half, split.to(torch.bfloat16))
+    assert float((split[rows.cuda()].double().cpu() - y64).abs().max()) / rms <= TOL
+    # the same products, associated differently: G + 8 fp32 roundings of 2^-24 each, of partial sums within a few rms
+    assert float((split - ordered).abs().max()) <= 2e-5 * rms
+
+
 @pytest.mark.parametrize("m,n,ldo", [(129, 1, 1), (130, 257, 257), (200, 1003, 1003), (300, 384, 390), (1030, 250, 251)])
 def test_gemm_fp32_result_any_pitch(gk, m, n, ldo):
     # fp32 rows of any pitch and alignment: boxes of 32 x 32 are stored through shared memory
