@@ -17,16 +17,16 @@ There is no CPU implementation in this package.
 import torch
 
 from . import _lib
-from .fp8_codec import (BLOCK, _device_for, _read_status, _reencode_on_device, _status_buffer, _stream_ptr,
-                        quantize_act_1x128)
+from .fp8_codec import (BLOCK, _device_for, _device_guard, _empty, _read_status, _reencode_on_device, _status_buffer,
+                        _stream_ptr, _unread_status_buffer, quantize_act_1x128)
 
 # Zero-initialised scratch per (device, stream).  The small-M schedule keeps per-tile arrival counters
 # there and returns them to zero, so one buffer serves every call issued on that stream.
 _workspaces = {}
 
 
-def _workspace(dev, nbytes):
-    key = (dev.index, _stream_ptr())
+def _workspace(dev, nbytes, stream=None):
+    key = (dev.index, _stream_ptr(dev) if stream is None else stream)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = torch.zeros(max(nbytes, 1), dtype=torch.uint8, device=dev)
@@ -62,6 +62,13 @@ def _group_major(a_scales, m, g):
         return a_scales, a_scales.stride(1)
     t = a_scales.t().contiguous()          # [G, M]
     return t, m
+
+
+def _new_output(m, n, dtype, dev):
+    """An [m, n] result and its row pitch: bf16 rows start on 16-byte boundaries."""
+    ldo = n if dtype == torch.float32 else (n + 7) // 8 * 8
+    out = _empty(m, ldo, dtype, dev)
+    return (out if ldo == n else out[:, :n]), ldo
 
 
 def _row_independent_schedule(m):
@@ -135,7 +142,7 @@ def gemm_block_fp8(a_codes, a_scales, w_codes, w_scales, bias=None, out=None, ou
             raise ValueError("bias with N elements required")
         bias = bias.to(device=dev, dtype=torch.float32).contiguous().view(-1)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         if k % 16 != 0:
             # TMA needs 16-byte row pitches: pad K with zero codes (zero contributes nothing).
             kp = (k + 15) // 16 * 16
@@ -145,22 +152,21 @@ def gemm_block_fp8(a_codes, a_scales, w_codes, w_scales, bias=None, out=None, ou
         sa, ldsa = _group_major(a_scales.to(dev), m, g)
         w_scales = w_scales.to(dev)
         if out is None:
-            ldo = n if out_dtype == torch.float32 else (n + 7) // 8 * 8
-            storage = torch.empty((m, ldo), dtype=out_dtype, device=dev)
-            out = storage[:, :n]
+            out, ldo = _new_output(m, n, out_dtype, dev)
         else:
             if (out.dtype != out_dtype or tuple(out.shape) != (m, n) or out.stride(1) != 1
                     or out.device != dev):
                 raise ValueError("out must be [M, N] of out_dtype with unit column stride on the operand device")
             ldo = out.stride(0)
-        ws_bytes = lib.bfp8_gemm_block128_workspace_bytes(m, n, k)
-        ws = _workspace(dev, ws_bytes) if ws_bytes else None
-        st = status if status is not None else _status_buffer(dev)
+        ws_bytes = lib.bfp8_gemm_block128_workspace_bytes(m, n, k) if m <= 128 else 0
+        stream = _stream_ptr(dev)
+        ws = _workspace(dev, ws_bytes, stream) if ws_bytes else None
+        st = status if status is not None else _status_buffer(dev) if check else _unread_status_buffer(dev)
         rc = lib.bfp8_gemm_block128_ex(
             a_codes.data_ptr(), lda, sa.data_ptr(), ldsa, w_codes.data_ptr(), ldw, w_scales.data_ptr(),
             bias.data_ptr() if bias is not None else None, out.data_ptr(),
             _lib.OUT_BF16 if out_dtype == torch.bfloat16 else _lib.OUT_F32, ldo, m, n, k,
-            ws.data_ptr() if ws is not None else None, ws_bytes, st.data_ptr() + 8, _stream_ptr(),
+            ws.data_ptr() if ws is not None else None, ws_bytes, st.data_ptr() + 8, stream,
             schedule, max_ctas, wait_limit_cycles)
         _lib.check(rc, "bfp8_gemm_block128")
         if check and _read_status(st)[1] & _lib.STATUS_WAIT_TIMEOUT:
@@ -195,7 +201,7 @@ def gemm_token_channel_fp8(a_codes, a_scales, w_codes, w_scales, bias=None, out=
             raise ValueError("bias with N elements required")
         bias = bias.to(device=dev, dtype=torch.float32).contiguous().view(-1)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         if k % 16 != 0:
             kp = (k + 15) // 16 * 16
             a_codes = torch.nn.functional.pad(a_codes.view(torch.uint8), (0, kp - k))
@@ -203,17 +209,17 @@ def gemm_token_channel_fp8(a_codes, a_scales, w_codes, w_scales, bias=None, out=
         a_scales = a_scales.to(dev).contiguous().view(-1)
         w_scales = w_scales.to(dev).contiguous().view(-1)
         if out is None:
-            ldo = n if out_dtype == torch.float32 else (n + 7) // 8 * 8
-            out = torch.empty((m, ldo), dtype=out_dtype, device=dev)[:, :n]
+            out, ldo = _new_output(m, n, out_dtype, dev)
         else:
             if out.dtype != out_dtype or tuple(out.shape) != (m, n) or out.stride(1) != 1 or out.device != dev:
                 raise ValueError("out must be [M, N] of out_dtype with unit column stride on the operand device")
             ldo = out.stride(0)
-        st = _status_buffer(dev)
+        st = _status_buffer(dev) if check else _unread_status_buffer(dev)
         rc = lib.bfp8_gemm_token_channel(
             a_codes.data_ptr(), a_codes.stride(0), a_scales.data_ptr(), w_codes.data_ptr(), w_codes.stride(0),
             w_scales.data_ptr(), bias.data_ptr() if bias is not None else None, out.data_ptr(),
-            _lib.OUT_BF16 if out_dtype == torch.bfloat16 else _lib.OUT_F32, ldo, m, n, k, st.data_ptr() + 8, _stream_ptr())
+            _lib.OUT_BF16 if out_dtype == torch.bfloat16 else _lib.OUT_F32, ldo, m, n, k, st.data_ptr() + 8,
+            _stream_ptr(dev))
         _lib.check(rc, "bfp8_gemm_token_channel")
         if check and _read_status(st)[1] & _lib.STATUS_WAIT_TIMEOUT:
             raise _lib.Bfp8Error(_WAIT_TIMEOUT_MSG)
@@ -256,7 +262,7 @@ def prepare_weight_swiglu(weight, scales, native_half=True):
     inter, k = codes.shape[0] // 2, codes.shape[1]
     dev = codes.device
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         src = codes.contiguous().view(torch.uint8)
         if k % 16 != 0:
             src = torch.nn.functional.pad(src, (0, (k + 15) // 16 * 16 - k))
@@ -295,23 +301,24 @@ def gemm_block_fp8_swiglu(a_codes, a_scales, w_codes, w_scales, bias=None, out=N
             raise ValueError("bias with 2 * I elements required")
         bias = bias.to(device=dev, dtype=torch.float32).contiguous().view(-1)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         if k % 16 != 0:
             a_codes = torch.nn.functional.pad(a_codes.view(torch.uint8), (0, w_codes.shape[1] - k))
         sa, ldsa = _group_major(a_scales.to(dev), m, g)
         w_scales = w_scales.to(dev)
         if out is None:
-            out = torch.empty((m, inter), dtype=torch.bfloat16, device=dev)
+            out = _empty(m, inter, torch.bfloat16, dev)
         elif (out.dtype != torch.bfloat16 or tuple(out.shape) != (m, inter) or out.stride(1) != 1 or out.device != dev):
             raise ValueError("out must be bf16 [M, I] with unit column stride on the operand device")
-        st = _status_buffer(dev)
+        st = _status_buffer(dev) if check else _unread_status_buffer(dev)
         ws_bytes = lib.bfp8_gemm_block128_workspace_bytes(m, n2, w_codes.shape[1]) if (small_m and m <= 128) else 0
-        ws = _workspace(dev, ws_bytes) if ws_bytes else None
+        stream = _stream_ptr(dev)
+        ws = _workspace(dev, ws_bytes, stream) if ws_bytes else None
         rc = lib.bfp8_gemm_block128_swiglu(
             a_codes.data_ptr(), a_codes.stride(0), sa.data_ptr(), ldsa, w_codes.data_ptr(), w_codes.stride(0),
             w_scales.data_ptr(), bias.data_ptr() if bias is not None else None, out.data_ptr(), out.stride(0),
             m, inter, w_codes.shape[1], ws.data_ptr() if ws is not None else None, ws_bytes, st.data_ptr() + 8,
-            _stream_ptr())
+            stream)
         _lib.check(rc, "bfp8_gemm_block128_swiglu")
         if check and _read_status(st)[1] & _lib.STATUS_WAIT_TIMEOUT:
             _workspaces.clear()
@@ -362,7 +369,7 @@ def reference(x, weight, scales, *, native_half=False, bias=None, out_dtype=torc
     lib = _lib.load()
     dev = _device_for(x, weight, scales)
     on_host = x.device.type == "cpu"
-    with torch.cuda.device(dev):
+    with _device_guard(dev):
         wd = weight.to(dev, non_blocking=True).contiguous()
         sd = scales.to(dev, non_blocking=True).contiguous()
         st = _status_buffer(dev)
