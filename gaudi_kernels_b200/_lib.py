@@ -32,6 +32,7 @@ SIGNATURES = {
     "bfp8_gemm_block128_workspace_bytes": (_sz, [_i64, _i64, _i64]),
     "bfp8_gemm_block128": (_int, [_ptr, _i64, _ptr, _i64, _ptr, _i64, _ptr, _ptr, _ptr, _int, _i64,
                                   _i64, _i64, _i64, _ptr, _sz, _ptr, _ptr]),
+    "bfp8_repitch_codes": (_int, [_ptr, _i64, _ptr, _ptr, _i64, _ptr, _i64, _i64, _ptr]),
     "bfp8_gemm_block128_ex": (_int, [_ptr, _i64, _ptr, _i64, _ptr, _i64, _ptr, _ptr, _ptr, _int, _i64,
                                      _i64, _i64, _i64, _ptr, _sz, _ptr, _ptr, _int, _int, _i64]),
     "bfp8_quant_act_token_bf16": (_int, [_ptr, _i64, _i64, _i64, _ptr, _i64, _ptr, _int, _ptr, _ptr]),

@@ -64,6 +64,19 @@ def _group_major(a_scales, m, g):
     return t, m
 
 
+def _with_pitch(lib, a_codes, w_codes, k, dev):
+    """The code rows with K zero-padded to a multiple of 16: TMA needs 16-byte row pitches, and zero contributes nothing.
+    w_codes may be None."""
+    kp = (k + 15) // 16 * 16
+    a = _empty(a_codes.shape[0], kp, torch.uint8, dev)
+    w = None if w_codes is None else _empty(w_codes.shape[0], kp, torch.uint8, dev)
+    rc = lib.bfp8_repitch_codes(a_codes.data_ptr(), a.shape[0], a.data_ptr(),
+                                None if w is None else w_codes.data_ptr(), 0 if w is None else w.shape[0],
+                                None if w is None else w.data_ptr(), k, kp, _stream_ptr(dev))
+    _lib.check(rc, "bfp8_repitch_codes")
+    return a, w
+
+
 def _new_output(m, n, dtype, dev):
     """An [m, n] result and its row pitch: bf16 rows start on 16-byte boundaries."""
     ldo = n if dtype == torch.float32 else (n + 7) // 8 * 8
@@ -144,10 +157,7 @@ def gemm_block_fp8(a_codes, a_scales, w_codes, w_scales, bias=None, out=None, ou
     lib = _lib.load()
     with _device_guard(dev):
         if k % 16 != 0:
-            # TMA needs 16-byte row pitches: pad K with zero codes (zero contributes nothing).
-            kp = (k + 15) // 16 * 16
-            a_codes = torch.nn.functional.pad(a_codes.view(torch.uint8), (0, kp - k))
-            w_codes = torch.nn.functional.pad(w_codes.view(torch.uint8), (0, kp - k))
+            a_codes, w_codes = _with_pitch(lib, a_codes, w_codes, k, dev)
         lda, ldw = a_codes.stride(0), w_codes.stride(0)
         sa, ldsa = _group_major(a_scales.to(dev), m, g)
         w_scales = w_scales.to(dev)
@@ -203,9 +213,7 @@ def gemm_token_channel_fp8(a_codes, a_scales, w_codes, w_scales, bias=None, out=
     lib = _lib.load()
     with _device_guard(dev):
         if k % 16 != 0:
-            kp = (k + 15) // 16 * 16
-            a_codes = torch.nn.functional.pad(a_codes.view(torch.uint8), (0, kp - k))
-            w_codes = torch.nn.functional.pad(w_codes.view(torch.uint8), (0, kp - k))
+            a_codes, w_codes = _with_pitch(lib, a_codes, w_codes, k, dev)
         a_scales = a_scales.to(dev).contiguous().view(-1)
         w_scales = w_scales.to(dev).contiguous().view(-1)
         if out is None:
@@ -303,7 +311,7 @@ def gemm_block_fp8_swiglu(a_codes, a_scales, w_codes, w_scales, bias=None, out=N
     lib = _lib.load()
     with _device_guard(dev):
         if k % 16 != 0:
-            a_codes = torch.nn.functional.pad(a_codes.view(torch.uint8), (0, w_codes.shape[1] - k))
+            a_codes, _ = _with_pitch(lib, a_codes, None, k, dev)
         sa, ldsa = _group_major(a_scales.to(dev), m, g)
         w_scales = w_scales.to(dev)
         if out is None:

@@ -121,6 +121,64 @@ extern "C" int bfp8_gemm_token_channel(const uint8_t* a_codes, int64_t lda, cons
                              status_dev, kDefaultWaitLimit, 0, static_cast<cudaStream_t>(stream));
 }
 
+// ---- code rows of any length, given the 16-byte pitch that TMA needs --------------------------------------
+
+namespace {
+// Both operands of a GEMM in one launch: K that is not a multiple of 16 would otherwise take a fill and a strided copy
+// for each (16.5 us of device time at M=777, K=1000, N=1003 before a GEMM of 11).  A thread writes one 16-byte vector of a
+// destination row from the five aligned words that hold its source bytes, shifted into place; vectors at the ends of
+// the source, and bytes at or beyond k, are formed byte by byte.
+__global__ void __launch_bounds__(256)
+repitch_kernel(const uint8_t* __restrict__ a, int64_t rows_a, uint8_t* __restrict__ dst_a, const uint8_t* __restrict__ w,
+               int64_t rows_w, uint8_t* __restrict__ dst_w, int64_t k, uint32_t vecs) {
+  // launched with programmatic stream serialization (see launch_overlapped)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int64_t vecs_a = rows_a * vecs, total = vecs_a + rows_w * vecs;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const bool first = i < vecs_a;
+    const int64_t j = first ? i : i - vecs_a;
+    const uint8_t* src = first ? a : w;
+    const int64_t bytes = (first ? rows_a : rows_w) * k;
+    const int64_t row = j / vecs, col = (j - row * vecs) * 16, from = row * k + col;
+    const int valid = static_cast<int>(k - col < 16 ? k - col : 16);
+    uint32_t v[4] = {0u, 0u, 0u, 0u};
+    const uint32_t skew = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(src) + from) & 3u);
+    if (from >= 4 && from + 20 <= bytes) {                       // the five words lie inside the source
+      const uint32_t* p = reinterpret_cast<const uint32_t*>(src + from - skew);
+      uint32_t x[5];
+#pragma unroll
+      for (int q = 0; q < 5; ++q) x[q] = __ldg(p + q);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        v[q] = __funnelshift_r(x[q], x[q + 1], skew * 8);
+        const int keep = valid - 4 * q;                          // bytes of this word that belong to the row
+        if (keep < 4) v[q] = keep <= 0 ? 0u : v[q] & ((1u << (8 * keep)) - 1u);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 16; ++q)
+        if (q < valid) v[q >> 2] |= static_cast<uint32_t>(src[from + q]) << (8 * (q & 3));
+    }
+    uint4* dst = reinterpret_cast<uint4*>(first ? dst_a : dst_w) + j;
+    *dst = make_uint4(v[0], v[1], v[2], v[3]);
+  }
+}
+}  // namespace
+
+extern "C" int bfp8_repitch_codes(const uint8_t* a_codes, int64_t m, uint8_t* a_out, const uint8_t* w_codes, int64_t n,
+                                  uint8_t* w_out, int64_t k, int64_t ld_out, void* stream) {
+  if (m < 0 || n < 0 || m + n <= 0 || k <= 0 || m > (1 << 30) || n > (1 << 30) || k > (1 << 30)) return BFP8_ERR_SHAPE;
+  if ((m > 0 && (!a_codes || !a_out)) || (n > 0 && (!w_codes || !w_out))) return BFP8_ERR_NULL;
+  if (ld_out != (k + 15) / 16 * 16) return BFP8_ERR_SHAPE;
+  if (!aligned(a_out, 16) || !aligned(w_out, 16)) return BFP8_ERR_ALIGN;
+  const int64_t vecs = ld_out / 16, want = ((m + n) * vecs + 255) / 256, cap = static_cast<int64_t>(sm_count()) * 16;
+  return launch_overlapped(repitch_kernel, dim3(static_cast<unsigned>(want < cap ? want : cap)), dim3(256), 0,
+                           static_cast<cudaStream_t>(stream), a_codes, m, a_out, w_codes, n, w_out, k,
+                           static_cast<uint32_t>(vecs));
+}
+
 // ---- gate/up GEMM with the SwiGLU step fused into its epilogue ---------------------------------------
 
 namespace {

@@ -138,6 +138,12 @@ int bfp8_gemm_block128(const uint8_t* a_codes, int64_t lda, const float* a_scale
                        uint32_t* status_dev, void* stream);
 
 
+/* Copies the rows of both operands of a GEMM, k bytes each and contiguous in the source, to rows of ld_out = k rounded up
+ * to 16 bytes, the rest zero (a code of 0 contributes nothing): the row pitch bfp8_gemm_* needs where k % 16 != 0.
+ * Sources may have any alignment, destinations start on 16 bytes; either operand may be absent (0 rows). */
+int bfp8_repitch_codes(const uint8_t* a_codes, int64_t m, uint8_t* a_out, const uint8_t* w_codes, int64_t n,
+                       uint8_t* w_out, int64_t k, int64_t ld_out, void* stream);
+
 /* Same as bfp8_gemm_block128 with tuning / diagnostic knobs (0 = default for each):
  *   schedule           0 automatic (beyond m = 128 the large-tile schedule, where few tiles meet a long K with the
  *                      K range of a tile summed in slices by a cluster of up to 8 CTAs); 1 large-tile schedule (one

@@ -229,6 +229,22 @@ def test_gemm_fp32_result_any_pitch(gk, m, n, ldo):
     assert torch.equal(out16, out.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (1, 3, 15), (5, 2, 17), (3, 4, 33), (130, 7, 1003), (2, 300, 130), (9, 0, 24), (64, 1, 2041)])
+def test_repitched_codes(gk, m, n, k):
+    # rows of any length from sources of any alignment; the last row ends where the allocation does
+    from gaudi_kernels_b200 import _lib
+    from gaudi_kernels_b200.block_fp8_gemm import _with_pitch
+    g = torch.Generator(device="cuda").manual_seed(k)
+    kp = (k + 15) // 16 * 16
+    for skew in range(4):
+        flat = torch.randint(0, 256, (skew + (m + n) * k,), generator=g, device="cuda", dtype=torch.uint8)
+        a, w = flat[skew:skew + m * k].view(m, k), flat[skew + m * k:].view(n, k)
+        got_a, got_w = _with_pitch(_lib.load(), a, w if n else None, k, flat.device)
+        for src, got in ((a, got_a), (w, got_w)):
+            if got is not None:
+                assert tuple(got.shape) == (src.shape[0], kp) and torch.equal(got[:, :k], src) and not bool(got[:, k:].any())
+
+
 def test_gemm_output_tail_is_untouched(gk):
     # sentinel columns right of N and rows below M must survive (out-of-bounds write check)
     m, k, n = 70, 256, 203
