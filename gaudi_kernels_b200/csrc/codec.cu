@@ -633,6 +633,40 @@ decode_block128_kernel(const uint8_t* __restrict__ codes, int64_t rows, int64_t 
   }
 }
 
+// bf16 results whose rows are whole vectors of 8: a thread decodes the same 8 columns of kDecodeRows consecutive rows, so that
+// it reads one scale, divides nothing, has all of its loads in flight before the first use, and stores a full 16 bytes each
+// time.  blockDim.x threads stand side by side along a row, blockDim.y groups of rows below one another.
+// HBM-bound: 8192 x 8192 45.1 -> 35.3 us (5.7 TB/s).  fp32 results, whose 16-byte stores are 4 codes, are faster in the kernel
+// above (54.0 against 57.0 us in this form).
+constexpr int kDecodeRows = 8;
+
+__global__ void __launch_bounds__(kDecodeThreads)
+decode_rows_bf16_kernel(const uint8_t* __restrict__ codes, int64_t rows, int64_t cols, int64_t ld,
+                        const float* __restrict__ scales, int col_blocks, uint16_t* __restrict__ out, int64_t ld_out) {
+  const int64_t r0 = (static_cast<int64_t>(blockIdx.x) * blockDim.y + threadIdx.y) * kDecodeRows;
+  const int64_t c = (static_cast<int64_t>(blockIdx.y) * blockDim.x + threadIdx.x) * 8;
+  if (r0 >= rows || c >= cols) return;
+  const uint8_t* p = codes + r0 * ld + c;
+  uint2 q[kDecodeRows];
+#pragma unroll
+  for (int i = 0; i < kDecodeRows; ++i)
+    if (r0 + i < rows) q[i] = __ldcs(reinterpret_cast<const uint2*>(p + i * ld));
+  const float s = __ldg(scales + (r0 >> 7) * col_blocks + (c >> 7));       // kDecodeRows divides 128
+#pragma unroll
+  for (int i = 0; i < kDecodeRows; ++i) {
+    if (r0 + i >= rows) break;
+    uint32_t v[4];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const uint32_t x = w == 0 ? q[i].x : q[i].y;
+      const float2 lo = e4m3x2_to_float2(x & 0xffffu), hi = e4m3x2_to_float2(x >> 16);
+      v[2 * w] = pack_bf16x2(__fmul_rn(lo.x, s), __fmul_rn(lo.y, s));
+      v[2 * w + 1] = pack_bf16x2(__fmul_rn(hi.x, s), __fmul_rn(hi.y, s));
+    }
+    __stcs(reinterpret_cast<uint4*>(out + (r0 + i) * ld_out + c), make_uint4(v[0], v[1], v[2], v[3]));
+  }
+}
+
 }  // namespace bfp8
 
 using namespace bfp8;
@@ -788,6 +822,19 @@ extern "C" int bfp8_decode_block128(const uint8_t* codes, int64_t rows, int64_t 
   const int cb = static_cast<int>((cols + 127) / 128);
   const bool vec = aligned(codes, 4) && ld % 4 == 0 && cols % 4 == 0 && ld_out % 4 == 0 &&
                    aligned(out, bf16 ? 8 : 16);
+  const int64_t per_row = cols / 8;
+  if (bf16 && aligned(codes, 8) && ld % 8 == 0 && cols % 8 == 0 && ld_out % 8 == 0 && aligned(out, 16) &&
+      per_row <= 65535LL * 32 && rows < (1LL << 33)) {
+    int x = 32;
+    while (x < per_row && x < kDecodeThreads) x *= 2;
+    const dim3 block(x, kDecodeThreads / x);
+    const int64_t per_cta = static_cast<int64_t>(block.y) * kDecodeRows;
+    const dim3 grid(static_cast<unsigned>((rows + per_cta - 1) / per_cta), static_cast<unsigned>((per_row + x - 1) / x));
+    decode_rows_bf16_kernel<<<grid, block, 0, static_cast<cudaStream_t>(stream)>>>(
+        codes, rows, cols, ld, scales, cb, static_cast<uint16_t*>(out), ld_out);
+    BFP8_CUDA_TRY(cudaGetLastError());
+    return BFP8_OK;
+  }
   const int64_t quads = rows * ((cols + 3) / 4);
   if ((quads + kDecodeThreads - 1) / kDecodeThreads > 2147483647LL) return BFP8_ERR_SHAPE;
   const int grid = static_cast<int>((quads + kDecodeThreads * kDecodePer - 1) / (kDecodeThreads * kDecodePer));

@@ -178,6 +178,20 @@ def test_decode_matches_oracle(gk, shape, dtype):
     assert np.array_equal(got.float().cpu().numpy(), want)
 
 
+# rows of whole vectors: 1 to 256 threads side by side, last groups of fewer than 8 rows, partly filled last CTAs, and widths
+# that are a whole number of vectors for one result type only
+@pytest.mark.parametrize("shape", [(1, 8), (7, 4), (129, 264), (9, 1032), (300, 2056), (17, 8200), (8, 12), (1025, 520)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_decode_rows_of_whole_vectors(gk, shape, dtype):
+    rng = np.random.default_rng(shape[0] + shape[1])
+    finite = np.array([c for c in range(256) if c & 0x7F != 0x7F], dtype=np.uint8)
+    codes = np.ascontiguousarray(finite[rng.integers(0, finite.size, size=shape)])
+    scales = rng.random(((shape[0] + 127) // 128, (shape[1] + 127) // 128), dtype=np.float32)
+    want = ref.decode_block128(codes, scales, out_bf16=dtype == torch.bfloat16)
+    got = gk.decode_e4m3(_fp8(codes), torch.from_numpy(scales).cuda(), out_dtype=dtype)
+    assert np.array_equal(got.float().cpu().numpy(), want)
+
+
 def test_decode_all_codes(gk):
     codes = np.arange(256, dtype=np.uint8).reshape(2, 128)
     got = gk.decode_e4m3(_fp8(codes), torch.ones((1, 1), device="cuda")).cpu().numpy().reshape(-1)
