@@ -112,8 +112,8 @@ extern "C" int bfp8_gemm_token_channel(const uint8_t* a_codes, int64_t lda, cons
   if (bias && !aligned(bias, 4)) return BFP8_ERR_ALIGN;
   if (out_dtype == BFP8_OUT_BF16 && (!aligned(out, 16) || ldo % 8 != 0)) return BFP8_ERR_ALIGN;
   if (out_dtype == BFP8_OUT_F32 && !aligned(out, 4)) return BFP8_ERR_ALIGN;
-  // one pass over W: the weight-streaming form (16: 24.3 -> 14.8 us at K=4096, N=14336; 64: 23.6 -> 19.7; at 128 rows its
-  // epilogue paces it and the large tiles are faster, 24.2 against 26.8)
+  // one pass over W: the weight-streaming form (K=4096, N=14336: 24.3 -> 14.8 us at 16 rows, 23.6 -> 18.6 at 64; its epilogue
+  // paces it beyond: 24.7 at 128 rows, where a pair of CTAs per large tile takes 20.4)
   if (m <= 64)
     return launch_gemm_smallm_token(a_codes, lda, a_scales, w_codes, ldw, w_scales, bias, out, out_dtype, ldo, m, n, k,
                                     status_dev, kDefaultWaitLimit, static_cast<cudaStream_t>(stream));

@@ -10,6 +10,8 @@
 // MMAs accumulate over all of K into one of two 256-column TMEM buffers, and the epilogue warps drain the
 // other buffer (scale, bias, bf16, TMA store) while the next tile's MMAs run.
 //
+// Large calls run as CTA pairs on 256 x 256 tiles, calls with few tiles as clusters that split K (see the kernel).
+//
 // Warp roles (384 threads): warps 0-7 epilogue (two warpgroups of 128 columns each), warp 8 TMA producer,
 // warp 9 TMEM owner + MMA issuer, warps 10-11 idle (setmaxnreg hands their registers to the epilogue).
 // Persistent, one CTA per SM; every barrier wait is bounded and raises BFP8_STATUS_WAIT_TIMEOUT.
@@ -28,26 +30,35 @@ namespace {
 constexpr int BM = 128;
 constexpr int BN = 256;
 constexpr int BK = 128;
-constexpr int kStages = 4;
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = (kEpiWarps + 4) * 32;
 constexpr int kTmemCols = 512;
-constexpr int kABytes = BM * BK;
-constexpr int kBBytes = BN * BK;
-constexpr int kStageBytes = kABytes + kBBytes;
+// The forms of the kernel: one CTA per tile; a cluster of CTAs that share the K range of a tile; two CTAs that share the
+// MMAs of a 256 x 256 tile.
+enum Form { kOne, kSplitK, kPair };
+
+template <Form F>
+struct Cfg {
+  static constexpr int kABytes = BM * BK;                            // this CTA's A rows
+  static constexpr int kBBytes = (F == kPair ? BN / 2 : BN) * BK;    // W rows, or half of the pair's
+  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kStages = F == kPair ? 6 : 4;                 // 192 KB either way
+  static constexpr int kTileRows = F == kPair ? 2 * BM : BM;
+};
 constexpr int kOutWarpBytes = 32 * 64 * 2;
 constexpr int kOutStageBytes = kEpiWarps * kOutWarpBytes;
 
 struct SmemTail {
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
+  uint64_t full[6];                // of the pair's first CTA in the pair form
+  uint64_t empty[6];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
 
-constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kOutStageBytes + sizeof(SmemTail);
+constexpr int kSmemBytes = 1024 + Cfg<kOne>::kStages * Cfg<kOne>::kStageBytes + kOutStageBytes + sizeof(SmemTail);
+static_assert(Cfg<kPair>::kStages * Cfg<kPair>::kStageBytes == Cfg<kOne>::kStages * Cfg<kOne>::kStageBytes, "one layout");
 
 struct Params {
   const float* a_scales;   // [M]
@@ -75,10 +86,19 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
 
 // kSplit: few tiles and a long K range, so p.split CTAs form a cluster, each accumulates an equal slice of the tile's K
 // blocks and the partial tiles are exchanged and added as split_exchange.cuh describes.  One tile per cluster.
-template <bool kOutBf16, bool kSplit>
+//
+// kPair: two CTAs of a cluster on one 256 x 256 tile.  What bounds the one-CTA form is the feed of its shared memory: 48 KB
+// per K block arrive at about 62 B/clk per SM (785 cycles per K block, the MMAs take 512).  A cta_group::2 MMA reads its
+// own A rows and half of the W rows from each CTA, 32 KB per CTA and K block.  The first CTA issues the MMAs, its `full`
+// barriers collect the TMA bytes of both CTAs and its `tmem_empty` barriers the epilogue warps of both; the commits are
+// multicast to both CTAs' `empty` and `tmem_full` barriers.
+template <bool kOutBf16, Form F>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                     const __grid_constant__ CUtensorMap tmap_out, const Params p) {
+  using C = Cfg<F>;
+  constexpr bool kSplit = F == kSplitK;
+  constexpr int kStages = C::kStages, kStageBytes = C::kStageBytes, kABytes = C::kABytes, kTileRows = C::kTileRows;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
@@ -90,10 +110,10 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int lane = threadIdx.x & 31;
   const int num_tiles = p.tiles_m * p.tiles_n;
   // this CTA's first tile, the distance to its next, and its K blocks [g_first, g_first + G) of each
-  const int cs = kSplit ? p.split : 1;
-  const int crank = kSplit ? static_cast<int>(blockIdx.x % cs) : 0;
-  const int tile0 = kSplit ? static_cast<int>(blockIdx.x / cs) : static_cast<int>(blockIdx.x);
-  const int tile_step = kSplit ? num_tiles : static_cast<int>(gridDim.x);
+  const int cs = kSplit ? p.split : F == kPair ? 2 : 1;
+  const int crank = F == kOne ? 0 : static_cast<int>(blockIdx.x % cs);
+  const int tile0 = F == kOne ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x / cs);
+  const int tile_step = kSplit ? num_tiles : static_cast<int>(F == kPair ? gridDim.x >> 1 : gridDim.x);
   const int g_first = kSplit ? static_cast<int>(static_cast<long long>(crank) * p.groups / cs) : 0;
   const int G = kSplit ? static_cast<int>(static_cast<long long>(crank + 1) * p.groups / cs) - g_first : p.groups;
 
@@ -104,14 +124,19 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(ptx::smem_u32(&tail->tmem_full[b]), 1);
-      ptx::mbar_init(ptx::smem_u32(&tail->tmem_empty[b]), kEpiWarps);
+      ptx::mbar_init(ptx::smem_u32(&tail->tmem_empty[b]), (F == kPair ? 2 : 1) * kEpiWarps);
     }
     tail->abort_flag = 0;
     ptx::fence_mbar_init();
   }
   if (warp == kEpiWarps + 1) {
-    ptx::tmem_alloc(ptx::smem_u32(&tail->tmem_base), kTmemCols);
-    ptx::tmem_relinquish();
+    if (F == kPair) {
+      ptx::tmem_alloc_pair(ptx::smem_u32(&tail->tmem_base), kTmemCols);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(ptx::smem_u32(&tail->tmem_base), kTmemCols);
+      ptx::tmem_relinquish();
+    }
   }
   if (warp == kEpiWarps && lane == 0) {
     ptx::prefetch_tensormap(&tmap_a);
@@ -120,6 +145,7 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   }
   ptx::tc_fence_before_sync();
   __syncthreads();
+  if (F == kPair) ptx::cluster_sync_all();          // both CTAs' barriers exist before any remote arrival
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
   // the set-up above touches no global memory and may overlap the previous kernel of the stream
@@ -141,17 +167,24 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (!ok) break;
             const uint32_t full = ptx::smem_u32(&tail->full[stage]);
             const uint32_t a_dst = smem_base + stage * kStageBytes;
-            ptx::mbar_arrive_expect_tx(full, kStageBytes);
-            ptx::tma_load_2d(a_dst, &tmap_a, full, (g_first + g) * BK, tm * BM);
-            ptx::tma_load_2d(a_dst + kABytes, &tmap_w, full, (g_first + g) * BK, tn * BN);
+            if (F == kPair) {
+              const uint32_t full0 = ptx::cluster_map(full, 0);
+              if (crank == 0) ptx::mbar_arrive_expect_tx(full, 2 * kStageBytes);
+              ptx::tma_load_2d_pair(a_dst, &tmap_a, full0, g * BK, tm * kTileRows + crank * BM);
+              ptx::tma_load_2d_pair(a_dst + kABytes, &tmap_w, full0, g * BK, tn * BN + crank * (BN / 2));
+            } else {
+              ptx::mbar_arrive_expect_tx(full, kStageBytes);
+              ptx::tma_load_2d(a_dst, &tmap_a, full, (g_first + g) * BK, tm * BM);
+              ptx::tma_load_2d(a_dst + kABytes, &tmap_w, full, (g_first + g) * BK, tn * BN);
+            }
             if (++stage == kStages) { stage = 0; phase ^= 1u; }
           }
         }
       }
     } else if (warp == kEpiWarps + 1) {
-      // ------------------------------------------------------------------ MMA issuer
-      if (lane == 0) {
-        constexpr uint32_t idesc = ptx::umma_idesc_e4m3(BM, BN);
+      // ------------------------------------------------------------------ MMA issuer (of the pair's first CTA)
+      if (lane == 0 && (F != kPair || crank == 0)) {
+        constexpr uint32_t idesc = ptx::umma_idesc_e4m3(kTileRows, BN);
         uint32_t stage = 0, phase = 0, it = 0;
         bool ok = true;
         for (int t = tile0; t < num_tiles && ok; t += tile_step, ++it) {
@@ -168,13 +201,17 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             const uint64_t a_desc = ptx::umma_desc_k128(a_addr);
             const uint64_t b_desc = ptx::umma_desc_k128(a_addr + kABytes);
 #pragma unroll
-            for (int k4 = 0; k4 < BK / 32; ++k4)
-              ptx::umma_f8(d, a_desc + 2u * k4, b_desc + 2u * k4, idesc, (g | k4) != 0);
-            ptx::umma_commit(ptx::smem_u32(&tail->empty[stage]));
+            for (int k4 = 0; k4 < BK / 32; ++k4) {
+              if (F == kPair) ptx::umma_f8_pair(d, a_desc + 2u * k4, b_desc + 2u * k4, idesc, (g | k4) != 0);
+              else ptx::umma_f8(d, a_desc + 2u * k4, b_desc + 2u * k4, idesc, (g | k4) != 0);
+            }
+            if (F == kPair) ptx::umma_commit_pair(ptx::smem_u32(&tail->empty[stage]));
+            else ptx::umma_commit(ptx::smem_u32(&tail->empty[stage]));
             if (++stage == kStages) { stage = 0; phase ^= 1u; }
           }
           if (!ok) break;
-          ptx::umma_commit(ptx::smem_u32(&tail->tmem_full[buf]));
+          if (F == kPair) ptx::umma_commit_pair(ptx::smem_u32(&tail->tmem_full[buf]));
+          else ptx::umma_commit(ptx::smem_u32(&tail->tmem_full[buf]));
         }
       }
     }
@@ -190,7 +227,7 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     for (int t = tile0; t < num_tiles && ok; t += tile_step, ++it) {
       int tm, tn;
       tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
-      const int row0 = tm * BM + quad * 32;
+      const int row0 = tm * kTileRows + (F == kPair ? crank * BM : 0) + quad * 32;
       const int row = row0 + lane;
       const int col0 = tn * BN + wg * 128;
       const bool row_ok = row < p.m;
@@ -254,7 +291,9 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           // every column of the buffer has been read: release it to the MMA warp
           ptx::tc_fence_before_sync();
           __syncwarp();
-          ptx::mbar_arrive_lane0(ptx::smem_u32(&tail->tmem_empty[buf]), lane);
+          const uint32_t bar = ptx::smem_u32(&tail->tmem_empty[buf]);
+          if (F == kPair) ptx::mbar_arrive_remote_lane0(ptx::cluster_map(bar, 0), lane);
+          else ptx::mbar_arrive_lane0(bar, lane);
         }
         if (kOutBf16) {
           const int box = c >> 1;                        // one TMA box = 64 columns = two chunks
@@ -316,12 +355,29 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   // ------------------------------------------------------------------ teardown
   ptx::tc_fence_before_sync();
   __syncthreads();
+  if (F == kPair) ptx::cluster_sync_all();          // the peer may still use this CTA's shared memory or barriers
   ptx::tc_fence_after_sync();
   ptx::idle_after_abort(abort_flag);
-  if (warp == kEpiWarps + 1) ptx::tmem_dealloc(tmem_base, kTmemCols);
+  if (warp == kEpiWarps + 1) {
+    if (F == kPair) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
+    else ptx::tmem_dealloc(tmem_base, kTmemCols);
+  }
   if (threadIdx.x == 0 && tail->abort_flag != 0) atomicOr(p.status, BFP8_STATUS_WAIT_TIMEOUT);
 }
 
+}  // namespace
+
+namespace {
+// Whether the pair form is the faster one: a wave of pairs takes 0.92 of a wave of single CTAs (M=4096, K=4096, N=14336:
+// 181 against 196 us, both 13 waves; M=8192, K=14336, N=4096: 326 / 355), but its tiles are twice as tall, so an odd number
+// of 128-row tiles, or few of them, can cost it a wave.  Where the K range is worth splitting the one-CTA form has that -
+// except that up to 128 rows a pair, half of it on padding rows, also gives a tile two CTAs to stream W, without the
+// exchange (M=128, K=4096, N=14336: 20.4 us; split in two 23.7, one CTA 22.7; with N=8192, K=8192 four slices 24.1, pairs 28.0).
+bool pair_is_faster(int64_t m, int64_t cols, int64_t groups, int sms) {
+  const int64_t one = (m + BM - 1) / BM * cols, two = (m + 2 * BM - 1) / (2 * BM) * cols;
+  const int64_t one_waves = (one + sms - 1) / sms, two_waves = (two + sms / 2 - 1) / (sms / 2);
+  return split_cluster_size(one, groups, sms) <= (m <= BM ? 2 : 1) && two_waves * 92 <= one_waves * 100;
+}
 }  // namespace
 
 int launch_gemm_channel(const uint8_t* a_codes, int64_t lda, const float* a_scales, const uint8_t* w_codes,
@@ -331,7 +387,10 @@ int launch_gemm_channel(const uint8_t* a_codes, int64_t lda, const float* a_scal
   alignas(64) CUtensorMap tmap_a, tmap_w, tmap_out;
   int rc = make_tensor_map_2d(&tmap_a, CU_TENSOR_MAP_DATA_TYPE_UINT8, a_codes, k, m, lda, BK, BM);
   if (rc != BFP8_OK) return rc;
-  rc = make_tensor_map_2d(&tmap_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, w_codes, k, n, ldw, BK, BN);
+  const int sms = sm_count();
+  const bool pair = max_ctas <= 0 && pair_is_faster(m, (n + BN - 1) / BN, (k + BK - 1) / BK, sms);
+  const int tile_rows = pair ? Cfg<kPair>::kTileRows : BM;
+  rc = make_tensor_map_2d(&tmap_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, w_codes, k, n, ldw, BK, pair ? BN / 2 : BN);
   if (rc != BFP8_OK) return rc;
   const bool bf16 = out_dtype == BFP8_OUT_BF16;
   if (bf16) {
@@ -349,12 +408,12 @@ int launch_gemm_channel(const uint8_t* a_codes, int64_t lda, const float* a_scal
   p.m = static_cast<int>(m);
   p.n = static_cast<int>(n);
   p.groups = static_cast<int>((k + BK - 1) / BK);
-  p.tiles_m = static_cast<int>((m + BM - 1) / BM);
+  p.tiles_m = static_cast<int>((m + tile_rows - 1) / tile_rows);
   p.tiles_n = static_cast<int>((n + BN - 1) / BN);
   p.wait_limit = wait_limit;
   p.status = status_dev;
   const int tiles = p.tiles_m * p.tiles_n;
-  int grid = sm_count();
+  int grid = pair ? sms / 2 : sms;                       // pairs, or CTAs
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (tiles < grid) grid = tiles;
   cudaLaunchAttribute attr[2];
@@ -367,9 +426,23 @@ int launch_gemm_channel(const uint8_t* a_codes, int64_t lda, const float* a_scal
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   p.split = 1;
-  const int want = max_ctas <= 0 ? split_cluster_size(tiles, p.groups, sm_count()) : 1;
+  if (pair) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+    cfg.gridDim = dim3(static_cast<unsigned>(grid * 2), 1, 1);
+    auto kern = bf16 ? gemm_channel_kernel<true, kPair> : gemm_channel_kernel<false, kPair>;
+    static DeviceFlags done[2];
+    rc = ensure_smem_limit(kern, kSmemBytes, done[bf16 ? 1 : 0]);
+    if (rc != BFP8_OK) return rc;
+    BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmap_a, tmap_w, tmap_out, p));
+    return BFP8_OK;
+  }
+  const int want = max_ctas <= 0 ? split_cluster_size(tiles, p.groups, sms) : 1;
   if (want > 1) {
-    auto kern = bf16 ? gemm_channel_kernel<true, true> : gemm_channel_kernel<false, true>;
+    auto kern = bf16 ? gemm_channel_kernel<true, kSplitK> : gemm_channel_kernel<false, kSplitK>;
     static DeviceFlags done[2];
     rc = ensure_smem_limit(kern, kSmemBytes, done[bf16 ? 1 : 0]);
     if (rc != BFP8_OK) return rc;
@@ -388,7 +461,7 @@ int launch_gemm_channel(const uint8_t* a_codes, int64_t lda, const float* a_scal
     }
     cfg.numAttrs = 1;
   }
-  auto kern = bf16 ? gemm_channel_kernel<true, false> : gemm_channel_kernel<false, false>;
+  auto kern = bf16 ? gemm_channel_kernel<true, kOne> : gemm_channel_kernel<false, kOne>;
   static DeviceFlags done[2];
   rc = ensure_smem_limit(kern, kSmemBytes, done[bf16 ? 1 : 0]);
   if (rc != BFP8_OK) return rc;

@@ -78,46 +78,13 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t cta) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
   return r;
 }
-// TMA tile load whose completion bytes are counted on a barrier that may live in the peer CTA.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish_pair() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void umma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// Arrive, once the MMAs issued so far have completed, on the barrier at this offset in both CTAs.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
-  const uint16_t mask = 3;
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(bar), "h"(mask) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar_cluster) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
-}
-// The same from lane 0 only, as a predicated instruction (the warp does not branch; see ptx::mbar_arrive_lane0).
-__device__ __forceinline__ void mbar_arrive_remote_lane0(uint32_t bar_cluster, int lane) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.eq.s32 p, %1, 0;\n\t"
-      "@p mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t}"
-      ::"r"(bar_cluster), "r"(lane) : "memory");
-}
+using ptx::mbar_arrive_remote_lane0;
+using ptx::tma_load_2d_pair;
+using ptx::tmem_alloc_pair;
+using ptx::tmem_dealloc_pair;
+using ptx::tmem_relinquish_pair;
+using ptx::umma_commit_pair;
+using ptx::umma_f8_pair;
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(

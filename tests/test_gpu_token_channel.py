@@ -80,10 +80,12 @@ def test_token_channel_gemm_matches_restatement(gk, m, k, n):
 
 # decode form: clusters of 8, 4 and 2 CTAs per tile, one CTA per tile (more tiles than half the SMs), two tiles per CTA; every
 # padded row count at its edges; fewer K blocks than MMA issuers; K and N that are not multiples of anything.
-# Beyond 128 rows: K slices over clusters of 2, 3 and more CTAs, ragged last slice and columns.
+# Beyond: K slices over clusters of 2, 3 and more CTAs, ragged last slice and columns.
 @pytest.mark.parametrize("m,k,n", [(1, 128, 128), (16, 2048, 640), (17, 1040, 4000), (128, 4096, 6000), (3, 384, 9610),
                                    (33, 640, 12344), (64, 1000, 19000), (65, 256, 9700), (128, 1152, 19003),
-                                   (129, 4096, 515), (300, 2192, 1032), (513, 5120, 2049)])
+                                   (129, 4096, 515), (300, 2192, 1032), (513, 5120, 2049),
+                                   # CTA pairs: a ragged last pair row and column, one K block, several tiles per pair
+                                   (257, 640, 2051), (400, 128, 300), (1300, 400, 9000), (2049, 272, 5000)])
 def test_token_channel_gemm_weight_streaming_and_split_forms(gk, m, k, n):
     g = torch.Generator().manual_seed(m * 5 + n)
     x = torch.randn((m, k), generator=g).to(torch.bfloat16)
