@@ -156,8 +156,8 @@ gemm_block128_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
-  // the set-up above touches no global memory and may overlap the previous kernel of the stream
-  ptx::griddep_launch_dependents();
+  // the set-up above touches no global memory and may overlap the previous kernel of the stream (see the launch)
+  if (kSplit || num_tiles <= static_cast<int>(gridDim.x)) ptx::griddep_launch_dependents();
   ptx::griddep_wait();
 
   if (warp >= kEpiWarps) {
@@ -626,6 +626,9 @@ int launch_gemm_large(const uint8_t* a_codes, int64_t lda, const float* a_scales
   rc = ensure_smem_limit(kern, kSmemBytes, done[inter > 0 ? 2 : (bf16 ? 1 : 0)]);
   if (rc != BFP8_OK) return rc;
   cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
+  // Programmatic launch is for calls of one wave, whose fixed costs count (M=256, K=4096, N=14336: 23.4 -> 21.6 us).  With
+  // several waves it made a prefill FFN (M=8192, K=4096, I=14336) slower, 1764 against 1738 us.
+  cfg.numAttrs = tiles <= grid ? 1 : 0;
   BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmap_a, tmap_w, tmap_out, pmaps, p));
   return BFP8_OK;
 }
