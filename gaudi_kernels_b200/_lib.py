@@ -13,6 +13,7 @@ STATUS_WAIT_TIMEOUT = 0x4
 STATUS_NONFINITE_INPUT = 0x8
 OUT_F32 = 0
 OUT_BF16 = 1
+SCHEDULE_FRESH_WEIGHT = 0x100
 
 _c = ctypes
 _i64, _ptr, _int, _sz = _c.c_int64, _c.c_void_p, _c.c_int, _c.c_size_t

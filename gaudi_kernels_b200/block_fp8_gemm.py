@@ -66,7 +66,7 @@ def _group_major(a_scales, m, g):
 
 def _with_pitch(lib, a_codes, w_codes, k, dev):
     """The code rows with K zero-padded to a multiple of 16: TMA needs 16-byte row pitches, and zero contributes nothing.
-    w_codes may be None."""
+    w_codes may be None.  The copies are fresh: a GEMM that reads w is enqueued with SCHEDULE_FRESH_WEIGHT."""
     kp = (k + 15) // 16 * 16
     a = _empty(a_codes.shape[0], kp, torch.uint8, dev)
     w = None if w_codes is None else _empty(w_codes.shape[0], kp, torch.uint8, dev)
@@ -128,7 +128,8 @@ def gemm_block_fp8(a_codes, a_scales, w_codes, w_scales, bias=None, out=None, ou
     bias     fp32 [N] or None;  out_dtype torch.bfloat16 (default) or torch.float32
     schedule 0 (default) chooses by size: weight streaming for M <= 128; beyond that 128 x 256 tiles, whose K range is
              summed in slices by several SMs where there are too few tiles to occupy the GPU.  1 large tiles with
-             K blocks added in order, 2 weight streaming, 3 CTA pairs
+             K blocks added in order, 2 weight streaming, 3 CTA pairs.  With | _lib.SCHEDULE_FRESH_WEIGHT the weight
+             codes were written by a kernel enqueued just before this call and are not taken to be at rest
     check    read the device status word after the launch (one synchronisation) and raise if a
              bounded wait expired; pass False on a latency-critical path together with `status`
     status   a buffer from new_status() that receives the kernel's status bits; several calls may share one.
@@ -158,6 +159,7 @@ def gemm_block_fp8(a_codes, a_scales, w_codes, w_scales, bias=None, out=None, ou
     with _device_guard(dev):
         if k % 16 != 0:
             a_codes, w_codes = _with_pitch(lib, a_codes, w_codes, k, dev)
+            schedule |= _lib.SCHEDULE_FRESH_WEIGHT
         lda, ldw = a_codes.stride(0), w_codes.stride(0)
         sa, ldsa = _group_major(a_scales.to(dev), m, g)
         w_scales = w_scales.to(dev)
@@ -406,7 +408,8 @@ def reference(x, weight, scales, *, native_half=False, bias=None, out_dtype=torc
                                                st.data_ptr() + 8, _stream_ptr())
             _lib.check(rc, "bfp8_quant_act_1x128_bf16")
             return gemm_block_fp8(a_codes, a_scales.t(), enc, sw, bias=bias, out=dev_out, out_dtype=out_dtype,
-                                  check=False, status=st, schedule=_row_independent_schedule(mr))
+                                  check=False, status=st,
+                                  schedule=_row_independent_schedule(mr) | _lib.SCHEDULE_FRESH_WEIGHT)
 
         if not on_host:
             dev_out = out if (out is not None and out.device.type == "cuda") else None

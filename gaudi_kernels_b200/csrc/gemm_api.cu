@@ -23,7 +23,7 @@ int launch_gemm_smallm(const uint8_t* a_codes, int64_t lda, const float* a_scale
                        const uint8_t* w_codes, int64_t ldw, const float* w_scales, const float* bias, void* out,
                        int out_dtype, int64_t ldo, int64_t m, int64_t n, int64_t k, void* workspace,
                        uint32_t* status_dev, long long wait_limit, int max_ctas, int inter, const SmallPush* push,
-                       cudaStream_t st);
+                       bool fresh_weight, cudaStream_t st);
 int launch_gemm_channel(const uint8_t* a_codes, int64_t lda, const float* a_scales, const uint8_t* w_codes,
                         int64_t ldw, const float* w_scales, const float* bias, void* out, int out_dtype, int64_t ldo,
                         int64_t m, int64_t n, int64_t k, uint32_t* status_dev, long long wait_limit, int max_ctas,
@@ -69,6 +69,8 @@ extern "C" int bfp8_gemm_block128_ex(const uint8_t* a_codes, int64_t lda, const 
   if (bias && !aligned(bias, 4)) return BFP8_ERR_ALIGN;
   if (out_dtype == BFP8_OUT_BF16 && (!aligned(out, 16) || ldo % 8 != 0)) return BFP8_ERR_ALIGN;
   if (out_dtype == BFP8_OUT_F32 && !aligned(out, 4)) return BFP8_ERR_ALIGN;
+  const bool fresh_weight = (schedule & BFP8_SCHEDULE_FRESH_WEIGHT) != 0;
+  schedule &= ~BFP8_SCHEDULE_FRESH_WEIGHT;
   if (schedule < 0 || schedule > 3 || (schedule == 2 && (m > kSmallMRows || !smallm_supported(n)))) return BFP8_ERR_SHAPE;
   const bool small = schedule == 2 || (schedule == 0 && m <= kSmallMRows && smallm_supported(n));
   const long long limit = wait_limit_cycles > 0 ? wait_limit_cycles : kDefaultWaitLimit;
@@ -79,7 +81,8 @@ extern "C" int bfp8_gemm_block128_ex(const uint8_t* a_codes, int64_t lda, const 
     if (!aligned(workspace, 256)) return BFP8_ERR_ALIGN;
     if (sm_count() > kMaxCtas) return BFP8_ERR_UNSUPPORTED;
     return launch_gemm_smallm(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, bias, out, out_dtype, ldo,
-                              m, n, k, workspace, status_dev, limit, max_ctas, /*inter=*/0, /*push=*/nullptr, st);
+                              m, n, k, workspace, status_dev, limit, max_ctas, /*inter=*/0, /*push=*/nullptr,
+                              fresh_weight, st);
   }
   if (schedule == 3)
     return launch_gemm_pair(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, bias, out, out_dtype, ldo, m, n, k,
@@ -238,7 +241,7 @@ extern "C" int bfp8_gemm_block128_swiglu(const uint8_t* a_codes, int64_t lda, co
     if (sm_count() > kMaxCtas) return BFP8_ERR_UNSUPPORTED;
     return launch_gemm_smallm(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, bias, out, BFP8_OUT_BF16, ldo, m,
                               2 * inter, k, workspace, status_dev, kDefaultWaitLimit, 0, static_cast<int>(inter),
-                              /*push=*/nullptr, static_cast<cudaStream_t>(stream));
+                              /*push=*/nullptr, /*fresh_weight=*/false, static_cast<cudaStream_t>(stream));
   }
   return launch_gemm_large(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, bias, out, BFP8_OUT_BF16, ldo,
                            m, 2 * inter, k, status_dev, kDefaultWaitLimit, 0, /*band=*/0, static_cast<int>(inter),
@@ -331,7 +334,7 @@ extern "C" int bfp8_gemm_block128_push(const uint8_t* a_codes, int64_t lda, cons
     sp.rows = t.rows;
     return launch_gemm_smallm(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, nullptr, const_cast<void*>(t.recv[rank]),
                               BFP8_OUT_BF16, n, m, n, k, workspace, status_dev, kDefaultWaitLimit, 0, /*inter=*/0, &sp,
-                              static_cast<cudaStream_t>(stream));
+                              /*fresh_weight=*/false, static_cast<cudaStream_t>(stream));
   }
   return launch_gemm_large(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, nullptr, const_cast<void*>(t.recv[rank]),
                            BFP8_OUT_BF16, n, m, n, k, status_dev, kDefaultWaitLimit, 0, /*band=*/0, /*inter=*/0, &t,

@@ -766,7 +766,7 @@ int launch_gemm_smallm(const uint8_t* a_codes, int64_t lda, const float* a_scale
                        const uint8_t* w_codes, int64_t ldw, const float* w_scales, const float* bias, void* out,
                        int out_dtype, int64_t ldo, int64_t m, int64_t n, int64_t k, void* workspace,
                        uint32_t* status_dev, long long wait_limit, int max_ctas, int inter, const SmallPush* push,
-                       cudaStream_t st) {
+                       bool fresh_weight, cudaStream_t st) {
   // inter > 0 selects the SwiGLU form: W has n = 2 * inter interleaved rows, `out` is bf16 [m, inter]
   // push != nullptr selects the push form: bf16 rows go to the receive areas of the GPUs that own them
   // max_ctas > 0 (a caller-imposed CTA limit, used by tests and by the entry point with the built-in scratch)
@@ -811,7 +811,8 @@ int launch_gemm_smallm(const uint8_t* a_codes, int64_t lda, const float* a_scale
     for (int o = 0; o < push->world; ++o) p.push_recv[o] = reinterpret_cast<uint16_t*>(const_cast<void*>(push->recv[o]));
   }
   p.cluster = max_ctas > 0 ? 0 : smallm_cluster_size(p.tiles, p.groups, sms);
-  p.w_early = g_weights_at_rest.load(std::memory_order_relaxed);
+  // the promise is about the caller's weights; one that a kernel before this launch has just written is not at rest
+  p.w_early = fresh_weight ? 0 : g_weights_at_rest.load(std::memory_order_relaxed);
   if (inter > 0) return dispatch<kSwiGLUForm>(mp, tmap_w, tmap_a, p, grid, st);
   return dispatch<kBlock>(mp, tmap_w, tmap_a, p, grid, st);
 }
@@ -914,7 +915,8 @@ extern "C" int bfp8_gemm_block128_noalloc(const uint8_t* a_codes, int64_t lda, c
   const size_t counter_bytes = static_cast<size_t>((n + BN - 1) / BN) * sizeof(uint32_t);
   BFP8_CUDA_TRY(cudaMemsetAsync(scratch, 0, counter_bytes, st));
   return launch_gemm_smallm(a_codes, lda, a_scales, ldsa, w_codes, ldw, w_scales, bias, out, out_dtype, ldo, m, n, k,
-                            scratch, status_dev, /*wait_limit=*/2000000000LL, kNoAllocMaxCtas, /*inter=*/0, /*push=*/nullptr, st);
+                            scratch, status_dev, /*wait_limit=*/2000000000LL, kNoAllocMaxCtas, /*inter=*/0, /*push=*/nullptr,
+                            /*fresh_weight=*/false, st);
 }
 
 #ifdef BFP8_TIMELINE

@@ -128,7 +128,7 @@ def reference_sharded(x_local, weight_local, scales_local, *, native_half=True, 
         if not on_host:
             y = gemm_block_fp8(a_codes, a_scales.t(), enc, sw, bias=bias_local,
                                out=out if (out is not None and out.device.type == "cuda") else None, check=False, status=st,
-                               schedule=_row_independent_schedule(m))
+                               schedule=_row_independent_schedule(m) | _lib.SCHEDULE_FRESH_WEIGHT)
         else:
             if out is None:
                 out = torch.empty((m, n_local), dtype=torch.bfloat16)
@@ -143,7 +143,7 @@ def reference_sharded(x_local, weight_local, scales_local, *, native_half=True, 
             for r0 in range(0, m, per):
                 r1 = min(m, r0 + per)
                 yr = gemm_block_fp8(a_codes[r0:r1], a_scales[:, r0:r1].t(), enc, sw, bias=bias_local, check=False, status=st,
-                                    schedule=_row_independent_schedule(r1 - r0))
+                                    schedule=_row_independent_schedule(r1 - r0) | _lib.SCHEDULE_FRESH_WEIGHT)
                 done = torch.cuda.Event()
                 done.record(main)
                 side.wait_event(done)

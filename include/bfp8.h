@@ -140,15 +140,21 @@ int bfp8_gemm_block128(const uint8_t* a_codes, int64_t lda, const float* a_scale
 
 /* Copies the rows of both operands of a GEMM, k bytes each and contiguous in the source, to rows of ld_out = k rounded up
  * to 16 bytes, the rest zero (a code of 0 contributes nothing): the row pitch bfp8_gemm_* needs where k % 16 != 0.
- * Sources may have any alignment, destinations start on 16 bytes; either operand may be absent (0 rows). */
+ * Sources may have any alignment, destinations start on 16 bytes; either operand may be absent (0 rows).  A GEMM enqueued
+ * behind it that reads w_out is given BFP8_SCHEDULE_FRESH_WEIGHT: w_out is not at rest yet. */
 int bfp8_repitch_codes(const uint8_t* a_codes, int64_t m, uint8_t* a_out, const uint8_t* w_codes, int64_t n,
                        uint8_t* w_out, int64_t k, int64_t ld_out, void* stream);
+
+#define BFP8_SCHEDULE_FRESH_WEIGHT 0x100   /* flag in the `schedule` argument below */
 
 /* Same as bfp8_gemm_block128 with tuning / diagnostic knobs (0 = default for each):
  *   schedule           0 automatic (beyond m = 128 the large-tile schedule, where few tiles meet a long K with the
  *                      K range of a tile summed in slices by a cluster of up to 8 CTAs); 1 large-tile schedule (one
  *                      CTA per 128x256 tile, K blocks added in order); 2 small-M weight-streaming
  *                      schedule (m <= 128); 3 CTA-pair schedule (clusters of two CTAs per 256x256 tile)
+ *                      | BFP8_SCHEDULE_FRESH_WEIGHT: the weight codes were written by a kernel enqueued just before this call
+ *                      (a copy made by bfp8_repitch_codes, a weight re-encoded for this one product); nothing of them is read
+ *                      before that kernel has ended, whatever bfp8_set_weights_at_rest promised
  *   max_ctas           upper bound on the persistent grid
  *   wait_limit_cycles  SM-clock budget of every internal barrier wait before WAIT_TIMEOUT is raised
  * The reference has no counterpart; its launch geometry is fixed per GUID in

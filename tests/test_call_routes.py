@@ -1,0 +1,79 @@
+"""Which C calls the Python entry points make, with which arguments, checked without a GPU.
+
+Fake tensors (device, shape and strides, no memory) go through the real entry points and a stand-in library records the
+calls, so rules about routes and flags are tested on the CPU, among them those whose breach would be a race on the device.
+"""
+
+import warnings
+
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+from gaudi_kernels_b200 import _lib, block_fp8_gemm
+
+
+class _Recorder:
+    """Stands for libbfp8.so: every function succeeds and is noted as (name, arguments)."""
+
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls.append((name, args))
+            return 0
+        return call
+
+    def named(self, name):
+        return [args for n, args in self.calls if n == name]
+
+
+@pytest.fixture
+def lib(monkeypatch):
+    rec = _Recorder()
+    monkeypatch.setattr(_lib, "load", lambda: rec)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 7, raising=False)
+    with warnings.catch_warnings(), FakeTensorMode():
+        warnings.simplefilter("ignore")                      # a fake tensor's data pointer is 0, and warns about it
+        yield rec
+
+
+def _operands(m, k, n):
+    groups = (k + 127) // 128
+    a = torch.empty((m, k), dtype=torch.uint8, device="cuda:0")
+    sa = torch.empty_strided((m, groups), (1, m), device="cuda:0")
+    w = torch.empty((n, k), dtype=torch.uint8, device="cuda:0")
+    ws = torch.empty(((n + 127) // 128, groups), device="cuda:0")
+    return a, sa, w, ws
+
+
+EX_SCHEDULE = 18                                             # position of `schedule` in bfp8_gemm_block128_ex
+
+
+@pytest.mark.parametrize("m", [1, 64, 128, 129])
+@pytest.mark.parametrize("k,schedule", [(1000, 0), (1003, 1), (1024, 0), (1008, 1)])
+def test_a_padded_copy_of_the_weight_is_declared_fresh(lib, m, k, schedule):
+    # K that is not a multiple of 16: the GEMM reads a copy which a kernel enqueued just before it writes; a weight declared
+    # at rest is read before that kernel has ended, so the copy must never be taken for one
+    a, sa, w, ws = _operands(m, k, 256)
+    status = torch.empty(4, dtype=torch.int32, device="cuda:0")
+    block_fp8_gemm.gemm_block_fp8(a, sa, w, ws, check=False, status=status, schedule=schedule)
+    copied = len(lib.named("bfp8_repitch_codes"))
+    assert copied == (1 if k % 16 else 0)
+    (args,) = lib.named("bfp8_gemm_block128_ex")
+    assert args[EX_SCHEDULE] == schedule | (_lib.SCHEDULE_FRESH_WEIGHT if copied else 0)
+
+
+@pytest.mark.parametrize("k", [1000, 1024])
+@pytest.mark.parametrize("native_half", [True, False])
+def test_reference_declares_its_weight_fresh(lib, monkeypatch, k, native_half):
+    # the weight is uploaded and re-encoded by the call itself
+    monkeypatch.setattr(block_fp8_gemm, "_read_status", lambda buf: (0, 0))
+    x = torch.empty((3, k), dtype=torch.bfloat16, device="cuda:0")
+    w = torch.empty((256, k), dtype=torch.float8_e4m3fn, device="cuda:0")
+    s = torch.empty((2, (k + 127) // 128), device="cuda:0")
+    block_fp8_gemm.reference(x, w, s, native_half=native_half)
+    (args,) = lib.named("bfp8_gemm_block128_ex")
+    assert args[EX_SCHEDULE] == _lib.SCHEDULE_FRESH_WEIGHT

@@ -9,7 +9,7 @@ import pytest
 import torch
 
 import gaudi_kernels_b200 as gk
-from gaudi_kernels_b200 import _lib
+from gaudi_kernels_b200 import _lib, block_fp8_gemm
 
 pytestmark = pytest.mark.gpu
 
@@ -96,6 +96,64 @@ def test_swiglu_chain_is_bit_identical_with_weights_at_rest(m, k, inter, at_rest
     plain = _chain(xs, w_codes, w_scales, swiglu=True)
     for i, (p, e) in enumerate(zip(plain, early)):
         assert torch.equal(p, e), "step %d differs" % i
+
+
+@pytest.mark.parametrize("k", [1000, 1003])
+@pytest.mark.parametrize("m", [1, 64, 128])
+@pytest.mark.parametrize("graph", [False, True])
+def test_weights_at_rest_of_any_row_length(m, k, graph):
+    """K that is not a multiple of 16: the GEMM reads a copy of the weight that the library makes in the same call, which is
+    not at rest.  Weights of one shape alternate, so that a copy read too early would be the other weight's."""
+    n = 14336
+    g = torch.Generator(device=DEV).manual_seed(31)
+    weights = [gk.prepare_weight(*gk.quantize_block128(torch.randn((n, k), generator=g, device=DEV) * (0.02 + 0.1 * i)))
+               for i in range(2)]
+    codes, scales = gk.quantize_act_1x128(torch.randn((m, k), generator=g, device=DEV).to(torch.bfloat16), native_half=True)
+    status = block_fp8_gemm.new_status(torch.device(DEV))
+
+    def enqueue():
+        return [gk.gemm_block_fp8(codes, scales, *weights[i % 2], check=False, status=status) for i in range(8)]
+
+    def results(at_rest):
+        prev = gk.set_weights_at_rest(at_rest)
+        try:
+            if not graph:
+                return [y.clone() for y in enqueue()]
+            side = torch.cuda.Stream()
+            with torch.cuda.stream(side):
+                enqueue()
+            torch.cuda.synchronize()
+            captured = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(captured, stream=side):
+                ys = enqueue()
+            captured.replay()
+            return [y.clone() for y in ys]
+        finally:
+            gk.set_weights_at_rest(prev)
+
+    plain, early = results(False), results(True)
+    torch.cuda.synchronize()
+    assert not block_fp8_gemm.wait_timed_out(status)
+    assert all(torch.equal(p, e) for p, e in zip(plain, early))
+    assert not torch.equal(plain[0], plain[1]) and torch.equal(plain[0], plain[2])
+
+
+@pytest.mark.parametrize("k", [1000, 1024])
+def test_reference_with_weights_at_rest(k):
+    """reference() re-encodes the weight it multiplies with in the same call."""
+    n = 2048
+    g = torch.Generator(device=DEV).manual_seed(37)
+    weights = [gk.quantize_block128(torch.randn((n, k), generator=g, device=DEV) * (0.02 + 0.1 * i)) for i in range(2)]
+    x = torch.randn((5, k), generator=g, device=DEV).to(torch.bfloat16)
+    results = []
+    for at_rest in (False, True):
+        prev = gk.set_weights_at_rest(at_rest)
+        try:
+            results.append([gk.reference(x, *weights[i % 2], native_half=True) for i in range(6)])
+        finally:
+            gk.set_weights_at_rest(prev)
+    assert all(torch.equal(p, e) for p, e in zip(*results))
+    assert not torch.equal(results[0][0], results[0][1])
 
 
 def test_graph_replay_with_weights_at_rest(at_rest):
