@@ -39,13 +39,17 @@ def shard_weight(w_codes, w_scales, world, rank):
 def gemm_sharded(a_codes, a_scales, w_codes_local, w_scales_local, bias_local=None, out=None, status=None):
     """This rank's [M, N_local] slice of the product (no communication).
 
+    Beyond M = 128 the K blocks are added in order whatever the size of the slice, so the slices have the bits of the whole
+    product in that order (gemm_block_fp8 with schedule=1, reference()), however many ranks share it.  gemm_block_fp8's
+    automatic schedule may sum a small slice's K range in pieces and rounds differently in fp32.
+
     The launch is not followed by a synchronisation.  Pass `status` (block_fp8_gemm.new_status(device), shared by
     as many calls as you like) and test it with block_fp8_gemm.wait_timed_out(status) once the step is complete:
     a kernel whose bounded wait expired reports it there and its output is invalid.
     """
-    from .block_fp8_gemm import gemm_block_fp8
+    from .block_fp8_gemm import _row_independent_schedule, gemm_block_fp8
     return gemm_block_fp8(a_codes, a_scales, w_codes_local, w_scales_local, bias=bias_local, out=out, check=False,
-                          status=status)
+                          status=status, schedule=_row_independent_schedule(a_codes.shape[0]))
 
 
 def gather_columns(local_out, group=None):

@@ -10,7 +10,7 @@ import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
-from gaudi_kernels_b200 import _lib, block_fp8_gemm
+from gaudi_kernels_b200 import _lib, block_fp8_gemm, sharded
 
 
 class _Recorder:
@@ -77,3 +77,12 @@ def test_reference_declares_its_weight_fresh(lib, monkeypatch, k, native_half):
     block_fp8_gemm.reference(x, w, s, native_half=native_half)
     (args,) = lib.named("bfp8_gemm_block128_ex")
     assert args[EX_SCHEDULE] == _lib.SCHEDULE_FRESH_WEIGHT
+
+
+@pytest.mark.parametrize("m,schedule", [(1, 0), (128, 0), (129, 1), (300, 1)])
+def test_column_slices_add_k_blocks_in_order(lib, m, schedule):
+    # a narrow slice has few tiles, which the automatic schedule may sum in slices of K: other bits than the whole product
+    a, sa, w, ws = _operands(m, 4096, 1024)
+    sharded.gemm_sharded(a, sa, w[256:512], ws[2:4])
+    (args,) = lib.named("bfp8_gemm_block128_ex")
+    assert args[EX_SCHEDULE] == schedule

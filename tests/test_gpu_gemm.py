@@ -413,3 +413,22 @@ def test_gemm_ffn70b_rank_slice_row_sample(gk):
     out_copy = gk.gemm_block_fp8(a_codes, a_scales, wl.contiguous(), sl.contiguous())
     assert torch.equal(out_view, out_copy)
 
+
+
+@pytest.mark.parametrize("m", [129, 300])
+def test_column_slices_have_the_bits_of_the_whole_product(gk, m):
+    # slices of 4096 to 512 columns: the automatic schedule would sum the narrow ones in slices of K
+    from gaudi_kernels_b200 import sharded
+    k, n = 4096, 4096
+    x, w, s, b = _random_problem(m, k, n, seed=m, bias=True)
+    a_codes, a_scales = gk.quantize_act_1x128(x.cuda(), native_half=True)
+    wc, ws = gk.prepare_weight(w, s, native_half=True)
+    whole = gk.gemm_block_fp8(a_codes, a_scales, wc, ws, bias=b.cuda(), schedule=1)
+    assert torch.equal(whole, gk.reference(x.cuda(), w.cuda(), s.cuda(), native_half=True, bias=b.cuda()))
+    for world in (1, 2, 4, 8):
+        parts = []
+        for rank in range(world):
+            lo, hi = sharded.shard_bounds(n, world, rank)
+            wl, sl = sharded.shard_weight(wc, ws, world, rank)
+            parts.append(sharded.gemm_sharded(a_codes, a_scales, wl, sl, bias_local=b[lo:hi].cuda()))
+        assert torch.equal(torch.cat(parts, 1), whole), world
