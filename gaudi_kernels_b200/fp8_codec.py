@@ -76,7 +76,7 @@ def _unread_status_buffer(device):
 
 
 def _read_status(buf):
-    lo, hi, status, _ = buf.tolist()       # synchronises with the launching stream
+    lo, hi, status = buf.tolist()[:3]      # synchronises with the launching stream; a caller's buffer may be longer
     return ((hi & 0xFFFFFFFF) << 32) | (lo & 0xFFFFFFFF), status & 0xFFFFFFFF
 
 

@@ -10,7 +10,7 @@ import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
-from gaudi_kernels_b200 import _lib, block_fp8_gemm, sharded
+from gaudi_kernels_b200 import _lib, block_fp8_gemm, fp8_codec, sharded
 
 
 class _Recorder:
@@ -86,3 +86,14 @@ def test_column_slices_add_k_blocks_in_order(lib, m, schedule):
     sharded.gemm_sharded(a, sa, w[256:512], ws[2:4])
     (args,) = lib.named("bfp8_gemm_block128_ex")
     assert args[EX_SCHEDULE] == schedule
+
+
+@pytest.mark.parametrize("words", [3, 4, 8])
+def test_status_buffers_of_any_length(words):
+    # a caller's own status buffer needs the three words that are read; what follows them does not matter
+    buf = torch.full((words,), -1, dtype=torch.int32)
+    buf[:3] = torch.tensor([-2, 1, _lib.STATUS_BAD_SCALE], dtype=torch.int32)
+    assert fp8_codec._read_status(buf) == ((1 << 32) | 0xFFFFFFFE, _lib.STATUS_BAD_SCALE)
+    assert not block_fp8_gemm.wait_timed_out(buf)
+    buf[2] |= _lib.STATUS_WAIT_TIMEOUT
+    assert block_fp8_gemm.wait_timed_out(buf)
