@@ -36,8 +36,9 @@ def _device_for(*tensors):
 # transpose 2.9 to 3.1), a status word that nobody can read left unzeroed (6.2, and a kernel).
 
 def _stream_ptr(dev=None):
-    """Raw handle of the current stream of `dev` (of the current device without it)."""
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if dev is None else dev.index)
+    """Raw handle of the current stream of `dev` (of the current device without it, or where it names no index)."""
+    index = None if dev is None else dev.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 class _NoContext:

@@ -4,13 +4,14 @@ Fake tensors (device, shape and strides, no memory) go through the real entry po
 calls, so rules about routes and flags are tested on the CPU, among them those whose breach would be a race on the device.
 """
 
+import contextlib
 import warnings
 
 import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
-from gaudi_kernels_b200 import _lib, block_fp8_gemm, fp8_codec, sharded
+from gaudi_kernels_b200 import _lib, block_fp8_gemm, fp8_codec, row_parallel, sharded
 
 
 class _Recorder:
@@ -29,12 +30,18 @@ class _Recorder:
         return [args for n, args in self.calls if n == name]
 
 
+def _raw_stream(index):
+    if not isinstance(index, int):
+        raise RuntimeError("a device index is required, as the real function does")
+    return 7
+
+
 @pytest.fixture
 def lib(monkeypatch):
     rec = _Recorder()
     monkeypatch.setattr(_lib, "load", lambda: rec)
     monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
-    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 7, raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", _raw_stream)
     with warnings.catch_warnings(), FakeTensorMode():
         warnings.simplefilter("ignore")                      # a fake tensor's data pointer is 0, and warns about it
         yield rec
@@ -97,3 +104,28 @@ def test_status_buffers_of_any_length(words):
     assert not block_fp8_gemm.wait_timed_out(buf)
     buf[2] |= _lib.STATUS_WAIT_TIMEOUT
     assert block_fp8_gemm.wait_timed_out(buf)
+
+
+class _Exchange:
+    """The parts of a PeerExchange that gemm_k_sharded uses, for a device named without an index."""
+
+    world, rank, nbytes, ptrs = 2, 0, 1 << 20, [0, 0]
+    device = torch.device("cuda")
+
+    def __init__(self, lib):
+        self.lib = lib
+        self.status = torch.empty(4, dtype=torch.int32, device="cuda:0")
+
+    def barrier(self):
+        pass
+
+
+def test_row_parallel_gemm_on_a_device_without_an_index(lib, monkeypatch):
+    # PeerExchange takes "cuda" for the current device; the decode bucket's workspace is kept per stream of that device
+    monkeypatch.setattr(torch.cuda, "device", lambda dev: contextlib.nullcontext())
+    monkeypatch.setattr(block_fp8_gemm, "_workspaces", {})
+    monkeypatch.setattr(_Recorder, "bfp8_gemm_block128_workspace_bytes", lambda self, m, n, k: 1024, raising=False)
+    a, sa, w, ws = _operands(8, 1024, 256)
+    row_parallel.gemm_k_sharded(a, sa, w, ws, _Exchange(lib))
+    assert len(lib.named("bfp8_gemm_block128_push")) == 1
+    assert list(block_fp8_gemm._workspaces) == [(None, 7)]
