@@ -86,23 +86,34 @@ inline int ensure_smem_limit(Kernel kernel, int bytes, DeviceFlags& done) {
   return BFP8_OK;
 }
 
-// Clusters of a kernel the current device can hold at once (0 on error), asked once per device and cluster size.  The
-// kernel's shared-memory limit has to be raised first and `cfg` must carry the cluster dimension.
+// Clusters of one kernel that a device holds at once, by device and cluster size: 0 not asked yet, else the number + 1.
 typedef std::atomic<int> ClusterCaps[64][9];
+
+// The number kept in `caps`, or what query(&number) answers.  An answer is kept; a failure (false) counts as 0 for this
+// call only, since which form a call takes decides the order of its sums.
+template <typename Query>
+inline int cached_clusters(ClusterCaps& caps, int dev, int cluster, Query query) {
+  if (cluster < 1 || cluster > 8) return 0;
+  const bool slot = dev >= 0 && dev < 64;
+  const int kept = slot ? caps[dev][cluster].load(std::memory_order_acquire) : 0;
+  if (kept > 0) return kept - 1;
+  int number = 0;
+  if (!query(&number) || number < 0) return 0;
+  if (slot) caps[dev][cluster].store(number + 1, std::memory_order_release);
+  return number;
+}
+
+// Clusters of a kernel the current device can hold at once (0 on error), asked once per device and cluster size; `caps`
+// belongs to this kernel.  Its shared-memory limit has to be raised first and `cfg` must carry the cluster dimension.
 template <typename Kernel>
 inline int max_active_clusters(Kernel kernel, const cudaLaunchConfig_t& cfg, int cluster, ClusterCaps& caps) {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cluster < 1 || cluster > 8) return 0;
-  const bool slot = dev >= 0 && dev < 64;
-  int cap = slot ? caps[dev][cluster].load(std::memory_order_acquire) : 0;
-  if (cap == 0) {
-    if (cudaOccupancyMaxActiveClusters(&cap, kernel, &cfg) != cudaSuccess) {
-      cudaGetLastError();                            // not left behind for the caller's next check
-      cap = 0;
-    }
-    if (slot) caps[dev][cluster].store(cap > 0 ? cap : -1, std::memory_order_release);
-  }
-  return cap > 0 ? cap : 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  return cached_clusters(caps, dev, cluster, [&](int* number) {
+    if (cudaOccupancyMaxActiveClusters(number, kernel, &cfg) == cudaSuccess) return true;
+    cudaGetLastError();                              // not left behind for the caller's next check
+    return false;
+  });
 }
 
 // Launch with the programmatic-stream-serialization attribute: the kernel may be scheduled while the previous

@@ -609,11 +609,11 @@ int launch_gemm_large(const uint8_t* a_codes, int64_t lda, const float* a_scales
     attr[1].val.clusterDim.y = 1;
     attr[1].val.clusterDim.z = 1;
     cfg.numAttrs = 2;
-    static ClusterCaps caps;
+    static ClusterCaps caps[2];
     for (int cs = want; cs > 1; --cs) {                // the largest cluster of which the device holds all `tiles` at once
       attr[1].val.clusterDim.x = static_cast<unsigned>(cs);
       cfg.gridDim = dim3(static_cast<unsigned>(tiles * cs), 1, 1);
-      if (max_active_clusters(kern, cfg, cs, caps) < tiles) continue;
+      if (max_active_clusters(kern, cfg, cs, caps[bf16 ? 1 : 0]) < tiles) continue;
       p.split = cs;
       BFP8_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmap_a, tmap_w, tmap_out, pmaps, p));
       return BFP8_OK;
