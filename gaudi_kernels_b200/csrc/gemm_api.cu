@@ -35,6 +35,9 @@ int launch_gemm_smallm_token(const uint8_t* a_codes, int64_t lda, const float* a
 size_t smallm_workspace_bytes(int64_t m, int64_t n, int max_ctas);
 int set_weights_at_rest(int on);
 bool smallm_supported(int64_t n);
+int smallm_cluster_size(int64_t tiles, int64_t groups, int sms);
+int large_k_split(int64_t m, int64_t n, int64_t groups, int sms);
+int channel_k_split(int64_t m, int64_t n, int64_t groups, int sms);
 }
 
 using namespace bfp8;
@@ -44,6 +47,9 @@ namespace {
 // launch returns with BFP8_STATUS_WAIT_TIMEOUT instead of hanging the device.
 constexpr long long kDefaultWaitLimit = 2000000000LL;
 constexpr int64_t kSmallMRows = 128;     // up to this many activation rows the weight-streaming schedule runs
+// The same of the token/channel GEMM, one pass over W (K=4096, N=14336: 24.3 -> 14.8 us at 16 rows, 23.6 -> 19.7 at 64; its
+// epilogue paces it beyond: 24.7 at 128 rows, where a pair of CTAs per large tile takes 20.4)
+constexpr int64_t kTokenStreamRows = 64;
 constexpr int kMaxCtas = 256;            // workspace is sized for this many CTAs, whatever the device has
 }
 
@@ -102,6 +108,17 @@ extern "C" int bfp8_gemm_block128(const uint8_t* a_codes, int64_t lda, const flo
 
 extern "C" int bfp8_set_weights_at_rest(int on) { return set_weights_at_rest(on); }
 
+extern "C" int bfp8_gemm_k_split(int64_t m, int64_t n, int64_t k, int token_channel, int sms) {
+  if (m <= 0 || n <= 0 || k <= 0) return BFP8_ERR_SHAPE;
+  if (sms <= 0) sms = sm_count();
+  const int64_t groups = (k + 127) / 128;
+  if (token_channel ? m <= kTokenStreamRows : m <= kSmallMRows && smallm_supported(n)) {
+    const int cluster = smallm_cluster_size((n + 127) / 128, groups, sms);
+    return cluster > 1 ? cluster : 1;
+  }
+  return token_channel ? channel_k_split(m, n, groups, sms) : large_k_split(m, n, groups, sms);
+}
+
 extern "C" int bfp8_gemm_token_channel(const uint8_t* a_codes, int64_t lda, const float* a_scales,
                                        const uint8_t* w_codes, int64_t ldw, const float* w_scales,
                                        const float* bias, void* out, int out_dtype, int64_t ldo,
@@ -115,9 +132,7 @@ extern "C" int bfp8_gemm_token_channel(const uint8_t* a_codes, int64_t lda, cons
   if (bias && !aligned(bias, 4)) return BFP8_ERR_ALIGN;
   if (out_dtype == BFP8_OUT_BF16 && (!aligned(out, 16) || ldo % 8 != 0)) return BFP8_ERR_ALIGN;
   if (out_dtype == BFP8_OUT_F32 && !aligned(out, 4)) return BFP8_ERR_ALIGN;
-  // one pass over W: the weight-streaming form (K=4096, N=14336: 24.3 -> 14.8 us at 16 rows, 23.6 -> 18.6 at 64; its epilogue
-  // paces it beyond: 24.7 at 128 rows, where a pair of CTAs per large tile takes 20.4)
-  if (m <= 64)
+  if (m <= kTokenStreamRows)
     return launch_gemm_smallm_token(a_codes, lda, a_scales, w_codes, ldw, w_scales, bias, out, out_dtype, ldo, m, n, k,
                                     status_dev, kDefaultWaitLimit, static_cast<cudaStream_t>(stream));
   return launch_gemm_channel(a_codes, lda, a_scales, w_codes, ldw, w_scales, bias, out, out_dtype, ldo, m, n, k,

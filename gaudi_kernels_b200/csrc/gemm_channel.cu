@@ -380,6 +380,12 @@ bool pair_is_faster(int64_t m, int64_t cols, int64_t groups, int sms) {
 }
 }  // namespace
 
+// CTAs that share a tile's K range (1 in the pair form, whose CTAs share the MMAs).
+int channel_k_split(int64_t m, int64_t n, int64_t groups, int sms) {
+  const int64_t cols = (n + BN - 1) / BN;
+  return pair_is_faster(m, cols, groups, sms) ? 1 : split_cluster_size((m + BM - 1) / BM * cols, groups, sms);
+}
+
 int launch_gemm_channel(const uint8_t* a_codes, int64_t lda, const float* a_scales, const uint8_t* w_codes,
                         int64_t ldw, const float* w_scales, const float* bias, void* out, int out_dtype, int64_t ldo,
                         int64_t m, int64_t n, int64_t k, uint32_t* status_dev, long long wait_limit, int max_ctas,

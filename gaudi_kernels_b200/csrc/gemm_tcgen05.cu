@@ -523,6 +523,11 @@ int split_cluster_size(int64_t tiles, int64_t groups, int sms) {
   return best;
 }
 
+// CTAs that share a tile's K range in a call that may split it.
+int large_k_split(int64_t m, int64_t n, int64_t groups, int sms) {
+  return split_cluster_size((m + BM - 1) / BM * ((n + BN - 1) / BN), groups, sms);
+}
+
 int launch_gemm_large(const uint8_t* a_codes, int64_t lda, const float* a_scales, int64_t ldsa,
                       const uint8_t* w_codes, int64_t ldw, const float* w_scales, const float* bias, void* out,
                       int out_dtype, int64_t ldo, int64_t m, int64_t n, int64_t k, uint32_t* status_dev,

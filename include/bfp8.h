@@ -189,6 +189,13 @@ int bfp8_gemm_token_channel(const uint8_t* a_codes, int64_t lda, const float* a_
                             const float* bias, void* out, int out_dtype, int64_t ldo,
                             int64_t m, int64_t n, int64_t k, uint32_t* status_dev, void* stream);
 
+/* How many CTAs share the K range of an output tile when the automatic schedule runs [m, k] x [n, k]^T on `sms` SMs (0: the
+ * current device's; with a number no device is touched): 1 means one CTA per tile (or a pair, or a list of tiles and
+ * parts of tiles per CTA for m <= 128), 2 to 8 a cluster that adds its members' partial sums in a fixed order, unless
+ * the device cannot hold that many clusters at once.  token_channel != 0 asks for bfp8_gemm_token_channel.  A negative
+ * BFP8_ERR_* code for sizes that are not positive.  The reference has no counterpart. */
+int bfp8_gemm_k_split(int64_t m, int64_t n, int64_t k, int token_channel, int sms);
+
 /* Declares, for the whole process, whether the weight operands (w_codes) of the decode-bucket GEMMs (m <= 128:
  * bfp8_gemm_block128, _ex, _swiglu, _push, _noalloc) are at rest.  These kernels are launched so that their
  * set-up overlaps the end of the previous kernel of the stream, and normally touch no global memory until that

@@ -184,11 +184,15 @@ def test_gemm_small_m_cluster_exchange(gk, m, k, n):
     assert torch.equal(out16, out.to(torch.bfloat16))
 
 
-@pytest.mark.parametrize("m,k,n", [(129, 4096, 255), (200, 2176, 1003), (256, 14336, 512), (300, 4096, 4096), (300, 2048, 2048),
-                                   (513, 3000, 1032), (640, 6144, 2816)])
+# (m, k, n) -> CTAs that share a tile's K range on 148 SMs: every size from 2 to 8 (test_host_rules.py asks the library), with
+# ragged rows, columns and last K block
+SPLIT_SHAPES = {(129, 4096, 255): 4, (200, 2176, 1003): 3, (256, 14336, 512): 7, (300, 4096, 4096): 3, (300, 2048, 2048): 2,
+                (513, 3000, 1032): 3, (640, 6144, 2816): 2, (150, 8600, 300): 5, (129, 11800, 250): 6, (140, 16300, 200): 8}
+
+
+@pytest.mark.parametrize("m,k,n", list(SPLIT_SHAPES))
 def test_gemm_split_k_matches_ordered_sum(gk, m, k, n):
-    # too few tiles for the GPU: clusters of 2 to 8 CTAs (these shapes reach 2, 3, 4, 5 and 6) sum slices of a tile's K range;
-    # ragged rows, columns and last K block
+    # too few tiles for the GPU: a cluster of CTAs sums slices of a tile's K range
     x, w, s, b = _random_problem(m, k, n, seed=m + k + n, bias=(m % 2 == 0))
     a_codes, a_scales = gk.quantize_act_1x128(x.cuda(), native_half=True)
     wc, ws = gk.prepare_weight(w, s, native_half=True)

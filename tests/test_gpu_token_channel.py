@@ -78,14 +78,19 @@ def test_token_channel_gemm_matches_restatement(gk, m, k, n):
             assert bool((num / den <= 0.01).all())          # the reference's device gate, fp8_hybrid_tpcsim_test.cpp:353-379
 
 
-# decode form: clusters of 8, 4 and 2 CTAs per tile, one CTA per tile (more tiles than half the SMs), two tiles per CTA; every
+# (m, k, n) -> CTAs that share a tile's K range on 148 SMs (test_host_rules.py asks the library).
+# Up to 64 rows: clusters of 8, 4 and 2 CTAs per tile, one CTA per tile (more tiles than half the SMs), two tiles per CTA; every
 # padded row count at its edges; fewer K blocks than MMA issuers; K and N that are not multiples of anything.
-# Beyond: K slices over clusters of 2, 3 and more CTAs, ragged last slice and columns.
-@pytest.mark.parametrize("m,k,n", [(1, 128, 128), (16, 2048, 640), (17, 1040, 4000), (128, 4096, 6000), (3, 384, 9610),
-                                   (33, 640, 12344), (64, 1000, 19000), (65, 256, 9700), (128, 1152, 19003),
-                                   (129, 4096, 515), (300, 2192, 1032), (513, 5120, 2049),
-                                   # CTA pairs: a ragged last pair row and column, one K block, several tiles per pair
-                                   (257, 640, 2051), (400, 128, 300), (1300, 400, 9000), (2049, 272, 5000)])
+# Beyond: K slices over clusters of 2 to 8 CTAs, ragged last slice and columns, and CTA pairs (1): a ragged last pair row and
+# column, one K block, several tiles per pair.
+FORMS = {(1, 128, 128): 1, (16, 2048, 640): 8, (17, 1040, 4000): 4, (5, 640, 9000): 2, (64, 1000, 9001): 2, (3, 384, 9610): 1,
+         (33, 640, 12344): 1, (64, 1000, 19000): 1, (65, 256, 9700): 1, (128, 1152, 19003): 1,
+         (128, 4096, 6000): 4, (129, 4096, 515): 4, (300, 2192, 1032): 3, (513, 5120, 2049): 3, (300, 2048, 2048): 2,
+         (150, 8600, 300): 5, (129, 11800, 250): 6, (256, 14336, 512): 7, (140, 16300, 200): 8,
+         (257, 640, 2051): 1, (400, 128, 300): 1, (1300, 400, 9000): 1, (2049, 272, 5000): 1}
+
+
+@pytest.mark.parametrize("m,k,n", list(FORMS))
 def test_token_channel_gemm_weight_streaming_and_split_forms(gk, m, k, n):
     g = torch.Generator().manual_seed(m * 5 + n)
     x = torch.randn((m, k), generator=g).to(torch.bfloat16)
@@ -104,8 +109,9 @@ def test_token_channel_gemm_weight_streaming_and_split_forms(gk, m, k, n):
         assert bool((buf[m:] == 0.75).all()) and bool((buf[:, n:] == 0.75).all())      # nothing written outside
         outs.append(out.clone())
     # fp32 sums of k products of E4M3 codes (exact): at most k + 4 roundings of 2^-24 of the largest partial sum, which a
-    # random walk keeps within a few rms; 2e-5 covers K = 5120 in any order of summation
-    assert float((outs[0].double().cpu() - y64).abs().max()) / rms <= 2e-5
+    # random walk keeps within a few rms; 2e-5 covers K = 5120 in any order of summation, longer sums have roundings in
+    # proportion
+    assert float((outs[0].double().cpu() - y64).abs().max()) / rms <= 2e-5 * max(1.0, k / 5120)
     assert torch.equal(outs[0], outs[1])                                               # fixed summation order
     assert torch.equal(outs[2], outs[0].to(torch.bfloat16))                            # same accumulator, RNE
 

@@ -2,7 +2,11 @@
 
 import subprocess
 
-from gaudi_kernels_b200 import build
+import pytest
+
+import test_gpu_gemm
+import test_gpu_token_channel
+from gaudi_kernels_b200 import _lib, build
 
 CLUSTER_CAPS = r"""
 #include <stdio.h>
@@ -42,3 +46,16 @@ def _run(source, tmp_path):
 def test_cluster_residency_is_kept_by_kernel_and_never_a_failure(tmp_path):
     res = _run(CLUSTER_CAPS, tmp_path)
     assert res.returncode == 0, res.stdout
+
+
+@pytest.mark.parametrize("token_channel,shapes", [(0, test_gpu_gemm.SPLIT_SHAPES), (1, test_gpu_token_channel.FORMS)])
+def test_the_gpu_tests_reach_every_cluster_size(token_channel, shapes):
+    build.build()
+    split = _lib.load().bfp8_gemm_k_split
+    for (m, k, n), want in shapes.items():
+        assert split(m, n, k, token_channel, 148) == want, (m, k, n)
+    large = {want for (m, k, n), want in shapes.items() if m > 128}
+    assert large >= {2, 3, 4, 5, 6, 7, 8}
+    if token_channel:
+        assert {want for (m, k, n), want in shapes.items() if m <= 64} >= {1, 2, 4, 8} and 1 in large
+    assert split(0, 1, 1, token_channel, 148) < 0
