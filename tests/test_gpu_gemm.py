@@ -436,3 +436,38 @@ def test_column_slices_have_the_bits_of_the_whole_product(gk, m):
             wl, sl = sharded.shard_weight(wc, ws, world, rank)
             parts.append(sharded.gemm_sharded(a_codes, a_scales, wl, sl, bias_local=b[lo:hi].cuda()))
         assert torch.equal(torch.cat(parts, 1), whole), world
+
+
+def test_gemm_as_the_first_cuda_work_of_a_thread(gk):
+    # a worker thread that has not launched anything yet has no driver context bound, and making tensor maps needs one
+    import threading
+    from gaudi_kernels_b200.block_fp8_gemm import new_status
+    status = new_status(torch.device("cuda", torch.cuda.current_device()))
+    calls = []
+    for m in (4, 300):
+        x, w, s, _ = _random_problem(m, 512, 512, seed=m)
+        a, sa = gk.quantize_act_1x128(x.cuda(), native_half=True)
+        at, st = gk.quantize_act_token(x.cuda())
+        wc, ws = gk.prepare_weight(w, s, native_half=True)
+        wg, wgs = gk.prepare_weight_swiglu(w, s)
+        rows = torch.rand(512, device="cuda")
+        calls += [lambda a=a, sa=sa, wc=wc, ws=ws: gk.gemm_block_fp8(a, sa, wc, ws, check=False),
+                  lambda a=a, sa=sa, wc=wc, ws=ws: gk.gemm_block_fp8(a, sa, wc, ws, check=False, status=status),
+                  lambda a=at, sa=st, wc=wc: gk.gemm_token_channel_fp8(a, sa, wc, rows, check=False),
+                  lambda a=a, sa=sa, wg=wg, wgs=wgs: gk.gemm_block_fp8_swiglu(a, sa, wg, wgs, check=False)]
+    want = [c() for c in calls]
+    torch.cuda.synchronize()
+    for i, call in enumerate(calls):
+        got = []
+
+        def work():
+            try:
+                got.append(call())
+            except Exception as e:                           # noqa: BLE001 - reported below
+                got.append(e)
+
+        t = threading.Thread(target=work)
+        t.start()
+        t.join()
+        assert isinstance(got[0], torch.Tensor), (i, got[0])
+        assert torch.equal(got[0], want[i]), i
