@@ -637,8 +637,11 @@ decode_block128_kernel(const uint8_t* __restrict__ codes, int64_t rows, int64_t 
 // it reads one scale, divides nothing, has all of its loads in flight before the first use, and stores a full 16 bytes each
 // time.  blockDim.x threads stand side by side along a row, blockDim.y groups of rows below one another.
 // HBM-bound: 8192 x 8192 45.1 -> 35.3 us (5.7 TB/s).  fp32 results, whose 16-byte stores are 4 codes, are faster in the kernel
-// above (54.0 against 57.0 us in this form).
+// above (54.0 against 57.0 us in this form).  So are rows of fewer than kDecodeRowsMinVecs vectors, which leave most of a warp's
+// lanes without one (kernel above / this form, us: 1 M rows of 8 columns 8.1 / 47.3, 512 K rows of 16 8.2 / 25.0, of 64
+// 24.1 / 25.2, of 72 26.8 / 25.5, of 96 34.5 / 26.0, of 128 45.2 / 32.3).
 constexpr int kDecodeRows = 8;
+constexpr int kDecodeRowsMinVecs = 9;
 
 __global__ void __launch_bounds__(kDecodeThreads)
 decode_rows_bf16_kernel(const uint8_t* __restrict__ codes, int64_t rows, int64_t cols, int64_t ld,
@@ -829,7 +832,7 @@ extern "C" int bfp8_decode_block128(const uint8_t* codes, int64_t rows, int64_t 
                    aligned(out, bf16 ? 8 : 16);
   const int64_t per_row = cols / 8;
   if (bf16 && aligned(codes, 8) && ld % 8 == 0 && cols % 8 == 0 && ld_out % 8 == 0 && aligned(out, 16) &&
-      per_row <= 65535LL * 32 && rows < (1LL << 33)) {
+      per_row >= kDecodeRowsMinVecs && per_row <= 65535LL * 32 && rows < (1LL << 33)) {
     int x = 32;
     while (x < per_row && x < kDecodeThreads) x *= 2;
     const dim3 block(x, kDecodeThreads / x);

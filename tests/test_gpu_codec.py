@@ -180,7 +180,9 @@ def test_decode_matches_oracle(gk, shape, dtype):
 
 # rows of whole vectors: 1 to 256 threads side by side, last groups of fewer than 8 rows, partly filled last CTAs, and widths
 # that are a whole number of vectors for one result type only
-@pytest.mark.parametrize("shape", [(1, 8), (7, 4), (129, 264), (9, 1032), (300, 2056), (17, 8200), (8, 12), (1025, 520)])
+# (narrow rows stay with the kernel for any shape: 8 to 64 columns)
+@pytest.mark.parametrize("shape", [(1, 8), (7, 4), (129, 264), (9, 1032), (300, 2056), (17, 8200), (8, 12), (1025, 520), (70000, 8),
+                                   (4097, 64), (4097, 72), (2051, 128)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_decode_rows_of_whole_vectors(gk, shape, dtype):
     rng = np.random.default_rng(shape[0] + shape[1])
