@@ -766,9 +766,10 @@ extern "C" int bfp8_quant_block128_f32(const float* w, int64_t rows, int64_t col
   return BFP8_OK;
 }
 
-// With fewer CTAs-for-rows than are resident at once (six per SM) each pass over a long row gets a CTA of its own; one CTA
-// walking all of its row's passes left the GPU part empty.  K=14336: 300 rows 5.9 -> 4.9 us, 512 rows 7.9 -> 6.1, 800 rows
-// 8.5 -> 7.9.
+// Up to six CTAs-for-rows per SM each pass over a long row gets a CTA of its own; one CTA walking all of its row's passes left
+// the GPU part empty.  Six is what is resident at once of the plain quantizer: K=14336, 300 rows 5.9 -> 4.9 us, 512 rows
+// 7.9 -> 6.1, 800 rows 8.5 -> 7.9.  Of the SiLU form four are, and the line stands at six there too: I=14336, 300 rows 13.3 ->
+// 9.4 us, 640 rows 17.5 -> 15.4, 740 rows 18.4 -> 17.0, 860 rows 20.3 -> 19.5; I=28672, 640 rows 32.6 -> 27.8, 740 33.1 -> 31.2.
 static int64_t act_split_rows() { return 6LL * sm_count(); }
 
 extern "C" int bfp8_quant_act_1x128_bf16(const uint16_t* x, int64_t m, int64_t k, int64_t ldx,

@@ -148,7 +148,9 @@ gemm_channel_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if (F == kPair) ptx::cluster_sync_all();          // both CTAs' barriers exist before any remote arrival
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
-  // the set-up above touches no global memory and may overlap the previous kernel of the stream
+  // the set-up above touches no global memory and may overlap the previous kernel of the stream.  Unlike in the block-scaled
+  // kernel this costs calls of several waves nothing: with its quantizer, M=4096, K=4096, N=14336 191.4 us against 192.3 in
+  // ordinary launches, M=8192 and K=14336 equal within the spread of the runs
   ptx::griddep_launch_dependents();
   ptx::griddep_wait();
 
