@@ -129,3 +129,23 @@ def test_row_parallel_gemm_on_a_device_without_an_index(lib, monkeypatch):
     row_parallel.gemm_k_sharded(a, sa, w, ws, _Exchange(lib))
     assert len(lib.named("bfp8_gemm_block128_push")) == 1
     assert list(block_fp8_gemm._workspaces) == [(None, 7)]
+
+
+@pytest.mark.parametrize("rows,schedule", [(3, 0), (200, 1)])
+def test_reference_sharded_declares_its_weight_fresh(lib, monkeypatch, rows, schedule):
+    class Enqueued(Exception):
+        pass
+
+    def all_reduce(*args, **kwargs):                         # the exchange of the status bits: every kernel is enqueued
+        raise Enqueued
+
+    monkeypatch.setattr(torch.cuda, "device", lambda dev: contextlib.nullcontext())
+    monkeypatch.setattr(sharded.dist, "get_world_size", lambda group=None: 1)
+    monkeypatch.setattr(sharded.dist, "all_gather_into_tensor", lambda *args, **kwargs: None)
+    monkeypatch.setattr(sharded.dist, "all_reduce", all_reduce)
+    x = torch.empty((rows, 1024), dtype=torch.bfloat16, device="cuda:0")
+    w = torch.empty((256, 1024), dtype=torch.float8_e4m3fn, device="cuda:0")
+    with pytest.raises(Enqueued):
+        sharded.reference_sharded(x, w, torch.empty((2, 8), device="cuda:0"))
+    (args,) = lib.named("bfp8_gemm_block128_ex")
+    assert args[EX_SCHEDULE] == schedule | _lib.SCHEDULE_FRESH_WEIGHT
